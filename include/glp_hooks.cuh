@@ -76,8 +76,17 @@ struct State {
 };
 
 constexpr uint32_t kFullMask = 0xffffffffu;
-constexpr int kSmemCap = 512; /* per warp; degrees <= kSmemCap/2 count in shared memory */
+constexpr int kSmemCap = 512; /* runs on graphs with a degree above kSmemCap/2 have the spill tables */
 constexpr uint32_t kErrProbe = 1u;
+
+constexpr int kPropThreads = 256;                 /* k_prop's block size */
+constexpr int kPropWarps = kPropThreads / 32;
+constexpr int kGroupDegree = 8;                   /* eight lanes per vertex up to here */
+constexpr int kWarpDegree = 128;                  /* a warp per vertex up to here; above, a block */
+constexpr int kBlockSlots = 2048;                 /* block table in shared memory (degree <= 1024) */
+constexpr int kWarpSlots = kBlockSlots / kPropWarps; /* = 2 * kWarpDegree */
+constexpr int kTurnSlots = 512;                   /* buckets that order the warps' adds */
+static_assert(kWarpSlots >= 2 * kWarpDegree && 2 * kWarpDegree <= kSmemCap, "table sizes");
 
 /* The 32-bit finaliser of MurmurHash3 (Appleby): slot of a key. */
 __device__ __forceinline__ uint32_t slot_hash(uint32_t k) {
@@ -95,104 +104,309 @@ __global__ void __launch_bounds__(256) k_pick(H h, int32_t n) {
   if (v < n) h.pick(v);
 }
 
-/* One warp per vertex.  The per-vertex table holds label+1 keys and FP64
- * frequencies: in shared memory up to degree kSmemCap/2, else in the global
- * spill region [2*off[v], 2*off[v] + cap) of gkeys/gvals (cap = the largest
- * power of two <= 2*degree, so it holds every distinct label). */
+/* Claims or finds the slot of `key` (not 0) among cap slots; cap when the
+ * table is full. */
+__device__ __forceinline__ uint32_t claim_slot(uint32_t* keys, uint32_t cap, uint32_t key) {
+  uint32_t slot = __umulhi(slot_hash(key), cap);
+  for (uint32_t probe = 0; probe < cap; ++probe) {
+    const uint32_t prev = atomicCAS(keys + slot, 0u, key);
+    if (prev == 0u || prev == key) return slot;
+    if (++slot == cap) slot = 0u;
+  }
+  return cap;
+}
+
+/* A scored label (l < 0: none); the larger score wins, then the larger label. */
+struct Scored {
+  double s;
+  int32_t l;
+};
+__device__ __forceinline__ void take_better(Scored& b, double s, int32_t l) {
+  if (l >= 0 && (b.l < 0 || s > b.s || (s == b.s && l > b.l))) {
+    b.s = s;
+    b.l = l;
+  }
+}
+template <int G>
+__device__ __forceinline__ Scored group_best(Scored b) {
+#pragma unroll
+  for (int o = G / 2; o >= 1; o >>= 1) {
+    const double os = __shfl_xor_sync(kFullMask, b.s, o);
+    const int32_t ol = __shfl_xor_sync(kFullMask, b.l, o);
+    take_better(b, os, ol);
+  }
+  return b;
+}
+
+/* The frequency of the lane's label within a chunk of 32 entries, summed in
+ * entry order; valid on the first lane holding the label (true there).  lab
+ * = -1: the lane has no entry.  sf: the warp's 32 words.  Each such lane
+ * walks the lanes that hold its label, so a chunk costs as many reads as its
+ * most frequent label has entries (one when all differ). */
+__device__ __forceinline__ bool chunk_freq(int32_t lab, double f, double* sf, double* sum) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  sf[lane] = f;
+  uint32_t m = __match_any_sync(kFullMask, (uint32_t)lab);
+  __syncwarp();
+  const bool lead = lab != -1 && lane == __ffs(m) - 1;
+  double s = 0.0;
+  if (lead)
+    for (; m; m &= m - 1u) s += sf[__ffs(m) - 1];
+  *sum = s;
+  return lead;
+}
+
+/* One propagation step.  A step reads each neighbour's label (and whatever
+ * LoadNeighbor asks for) at random, so it is bound by the latency of those
+ * reads and by the ordered FP64 sums; the split keeps every warp loading:
+ *   degree 0..8     eight lanes per vertex, four vertices per warp and round,
+ *                   two rounds' loads in flight; frequencies by shuffles;
+ *   degree 9..32    a warp per vertex, four vertices' entries loaded before
+ *                   the first is summed; one chunk holds the whole row, so
+ *                   its sums are the final frequencies and need no table;
+ *   degree 33..128  a warp per vertex, the whole row loaded first, then a
+ *                   per-warp shared table of two slots an entry;
+ *   above           a block per vertex, eight chunks at a time: every warp
+ *                   sums its chunk, then the adds to a label's frequency go
+ *                   in chunk order -- each leader notes its warp in the
+ *                   turn bucket of its slot and adds after as many barriers
+ *                   as lower warps share the bucket (usually none).  Tables
+ *                   in shared memory up to degree 1024, else in the vertex's
+ *                   own spill region [2*off[v], 2*off[v+1]) of gkeys/gvals.
+ * Vertices are dealt to blocks and warps with the grid as the stride, so
+ * that the neighbouring large rows of a degree-sorted graph land on
+ * different SMs; every phase scans the offsets for its degrees (8 bytes a
+ * vertex, cheaper than keeping lists in the public state).  Measured on one
+ * B200, R-MAT scale 20 (31.7 M entries), degree-normalised votes, ten steps:
+ * 32 ms; 640 ms with one warp per vertex of any degree, 512 slots cleared and
+ * scanned for each and full-warp shuffle sums. */
 template <class H>
-__global__ void __launch_bounds__(128) k_prop(H h, const State st, uint32_t* gkeys, double* gvals,
-                                              unsigned long long* changed, uint32_t* err) {
-  constexpr int NW = 4;
-  __shared__ uint32_t skeys[NW][kSmemCap];
-  __shared__ double svals[NW][kSmemCap];
+__global__ void __launch_bounds__(kPropThreads, 4) k_prop(H h, const State st, uint32_t* gkeys, double* gvals,
+                                                          unsigned long long* changed, uint32_t* err) {
+  __shared__ double svals[kBlockSlots]; /* the block's table, or one slice per warp */
+  __shared__ uint32_t skeys[kBlockSlots];
+  __shared__ uint32_t sturn[2][kTurnSlots];
+  __shared__ double sf[kPropWarps][32];
+  __shared__ Scored sred[kPropWarps];
+  __shared__ int32_t slist[kPropThreads];
+  __shared__ int32_t sn;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int32_t v = blockIdx.x * NW + warp; v < st.n; v += gridDim.x * NW) {
-    const int32_t b = st.off[v], e = st.off[v + 1], d = e - b;
-    if (d == 0) {
-      if (lane == 0) {
-        const int32_t l = st.L[v];
-        st.Lnext[v] = l;
-        h.update(v, l, -INFINITY);
+  const int64_t nb = gridDim.x, nw = nb * kPropWarps;
+  uint32_t nchanged = 0; /* this thread's */
+  bool full = false;
+  auto settle = [&](int32_t v, const Scored& b) {
+    st.Lnext[v] = b.l;
+    h.update(v, b.l, b.s);
+    nchanged += b.l != st.L[v] ? 1u : 0u;
+  };
+
+  /* above kWarpDegree: a block per vertex */
+  for (int i = threadIdx.x; i < 2 * kTurnSlots; i += kPropThreads) (&sturn[0][0])[i] = 0u;
+  int par = 0;
+  for (int64_t v0 = blockIdx.x; v0 < st.n; v0 += nb * kPropThreads) { /* block-uniform */
+    if (threadIdx.x == 0) sn = 0;
+    __syncthreads();
+    const int64_t vt = v0 + threadIdx.x * nb;
+    if (vt < st.n && st.off[vt + 1] - st.off[vt] > kWarpDegree) slist[atomicAdd(&sn, 1)] = (int32_t)vt;
+    __syncthreads();
+    const int32_t nlist = sn;
+    for (int32_t k = 0; k < nlist; ++k) {
+      const int32_t v = slist[k];
+      const int32_t b = st.off[v];
+      const uint32_t d = (uint32_t)(st.off[v + 1] - b), cap = 2u * d;
+      const bool spill = cap > (uint32_t)kBlockSlots;
+      uint32_t* keys = spill ? gkeys + 2ll * b : skeys;
+      double* vals = spill ? gvals + 2ll * b : svals;
+      for (uint32_t s = threadIdx.x; s < cap; s += kPropThreads) {
+        keys[s] = 0u;
+        vals[s] = 0.0;
       }
-      continue; /* warp-uniform */
-    }
-    uint32_t* keys;
-    double* vals;
-    uint32_t cap;
-    if (d <= kSmemCap / 2) {
-      keys = skeys[warp];
-      vals = svals[warp];
-      cap = kSmemCap;
-    } else {
-      cap = 1;
-      while (cap * 2 <= 2u * (uint32_t)d) cap *= 2;
-      keys = gkeys + 2ll * b;
-      vals = gvals + 2ll * b;
-    }
-    for (uint32_t s = lane; s < cap; s += 32) {
-      keys[s] = 0;
-      vals[s] = 0.0;
-    }
-    __syncwarp();
-    for (int32_t j0 = b; j0 < e; j0 += 32) {
-      const int32_t j = j0 + lane;
-      int32_t lab = -1;
-      double f = 0.0;
-      if (j < e) h.load(v, st.cols[j], j, &lab, &f);
-      const uint32_t m = __match_any_sync(kFullMask, (uint32_t)lab);
-      /* entry-ordered sum over the lanes holding the same label */
-      double s = 0.0;
-      for (int k = 0; k < 32; ++k) {
-        const double x = __shfl_sync(kFullMask, f, k);
-        if ((m >> k) & 1u) s += x;
-      }
-      if (j < e && lane == __ffs(m) - 1) {
-        const uint32_t key = (uint32_t)lab + 1u;
-        uint32_t slot = slot_hash(key) & (cap - 1);
-        bool done = false;
-        for (uint32_t probe = 0; probe < cap; ++probe) {
-          const uint32_t prev = atomicCAS(&keys[slot], 0u, key);
-          if (prev == 0u || prev == key) {
-            vals[slot] += s; /* one writer per label per chunk; chunks in order */
-            done = true;
-            break;
-          }
-          slot = (slot + 1) & (cap - 1);
+      __syncthreads();
+      for (uint32_t i0 = 0; i0 < d; i0 += 4 * kPropThreads) {
+        int32_t lab[4];
+        double f[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t i = i0 + q * kPropThreads + threadIdx.x;
+          lab[q] = -1;
+          f[q] = 0.0;
+          if (i < d) h.load(v, st.cols[b + i], b + (int64_t)i, &lab[q], &f[q]);
         }
-        if (!done) atomicOr(err, kErrProbe);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (d - i0 <= q * kPropThreads) break; /* block-uniform */
+          double s;
+          const bool lead = chunk_freq(lab[q], f[q], sf[warp], &s);
+          uint32_t slot = cap;
+          if (lead) {
+            slot = claim_slot(keys, cap, (uint32_t)lab[q] + 1u);
+            full = full || slot == cap;
+          }
+          const bool add = slot < cap;
+          uint32_t* turn = &sturn[par][slot & (kTurnSlots - 1)];
+          if (add) atomicOr(turn, 1u << warp);
+          __syncthreads();
+          const int rank = add ? __popc(*turn & ((1u << warp) - 1u)) : -1;
+          for (int r = 0;; ++r) {
+            if (rank == r) vals[slot] += s;
+            if (!__syncthreads_or(rank > r)) break;
+          }
+          if (add) *turn = 0u; /* the next chunk uses the other bucket set */
+          par ^= 1;
+        }
+      }
+      Scored best{-INFINITY, -1};
+      for (uint32_t s = threadIdx.x; s < cap; s += kPropThreads) {
+        const uint32_t key = keys[s];
+        if (key) {
+          const int32_t l = (int32_t)(key - 1u);
+          take_better(best, h.score(v, l, vals[s]), l);
+        }
+      }
+      best = group_best<32>(best);
+      if (lane == 0) sred[warp] = best;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int w = 1; w < kPropWarps; ++w) take_better(best, sred[w].s, sred[w].l);
+        settle(v, best);
+      }
+    }
+    __syncthreads(); /* the list is read no more */
+  }
+
+  /* 9..kWarpDegree: a warp per vertex */
+  uint32_t* wkeys = skeys + warp * kWarpSlots;
+  double* wvals = svals + warp * kWarpSlots;
+  for (int64_t v0 = warp * nb + blockIdx.x; v0 < st.n; v0 += 32 * nw) {
+    const int64_t vt = v0 + lane * nw;
+    int32_t vb = 0, vd = 0;
+    if (vt < st.n) {
+      vb = st.off[vt];
+      vd = st.off[vt + 1] - vb;
+    }
+    uint32_t one = __ballot_sync(kFullMask, vd > kGroupDegree && vd <= 32);
+    while (one) { /* four rows of one chunk each */
+      int32_t v[4], lab[4];
+      double f[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int src = one ? __ffs(one) - 1 : 0;
+        v[q] = one ? (int32_t)(v0 + src * nw) : -1;
+        one &= one - 1u;
+        const int32_t b = __shfl_sync(kFullMask, vb, src), d = __shfl_sync(kFullMask, vd, src);
+        lab[q] = -1;
+        f[q] = 0.0;
+        if (v[q] >= 0 && lane < d) h.load(v[q], st.cols[b + lane], b + lane, &lab[q], &f[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (v[q] < 0) break; /* warp-uniform */
+        double s;
+        Scored best{-INFINITY, -1};
+        if (chunk_freq(lab[q], f[q], sf[warp], &s)) take_better(best, h.score(v[q], lab[q], s), lab[q]);
+        best = group_best<32>(best);
+        if (lane == 0) settle(v[q], best);
+      }
+    }
+    uint32_t many = __ballot_sync(kFullMask, vd > 32 && vd <= kWarpDegree);
+    for (; many; many &= many - 1u) {
+      const int src = __ffs(many) - 1;
+      const int32_t v = (int32_t)(v0 + src * nw);
+      const int32_t b = __shfl_sync(kFullMask, vb, src), d = __shfl_sync(kFullMask, vd, src);
+      int32_t lab[4];
+      double f[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int32_t i = 32 * q + lane;
+        lab[q] = -1;
+        f[q] = 0.0;
+        if (i < d) h.load(v, st.cols[b + i], b + i, &lab[q], &f[q]);
+      }
+      const uint32_t cap = 2u * (uint32_t)d;
+      for (uint32_t s = lane; s < cap; s += 32) {
+        wkeys[s] = 0u;
+        wvals[s] = 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (32 * q >= d) break; /* warp-uniform */
+        double s;
+        if (chunk_freq(lab[q], f[q], sf[warp], &s)) { /* its barriers order the chunks' adds */
+          const uint32_t slot = claim_slot(wkeys, cap, (uint32_t)lab[q] + 1u);
+          if (slot < cap) wvals[slot] += s;
+          else full = true;
+        }
       }
       __syncwarp();
-    }
-    /* score every distinct label on its final frequency */
-    double bs = -INFINITY;
-    int32_t bl = -1;
-    for (uint32_t s = lane; s < cap; s += 32) {
-      const uint32_t key = keys[s];
-      if (key) {
-        const int32_t l = (int32_t)(key - 1u);
-        const double sc = h.score(v, l, vals[s]);
-        if (bl < 0 || sc > bs || (sc == bs && l > bl)) {
-          bs = sc;
-          bl = l;
+      Scored best{-INFINITY, -1};
+      for (uint32_t s = lane; s < cap; s += 32) {
+        const uint32_t key = wkeys[s];
+        if (key) {
+          const int32_t l = (int32_t)(key - 1u);
+          take_better(best, h.score(v, l, wvals[s]), l);
         }
+      }
+      best = group_best<32>(best);
+      if (lane == 0) settle(v, best);
+      __syncwarp(); /* the table is cleared for the next vertex */
+    }
+  }
+
+  /* 0..kGroupDegree: eight lanes per vertex */
+  const int gl = lane & 7;
+  for (int64_t w0 = (int64_t)blockIdx.x * kPropWarps + warp; w0 * 8 < st.n; w0 += nw) {
+    int32_t v[2], lab[2];
+    double f[2];
+    bool mine[2], row[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int64_t vt = w0 * 8 + 4 * q + (lane >> 3);
+      v[q] = (int32_t)vt;
+      lab[q] = -1;
+      f[q] = 0.0;
+      mine[q] = row[q] = false;
+      if (vt < st.n) {
+        const int32_t b = st.off[vt], d = st.off[vt + 1] - b;
+        mine[q] = d <= kGroupDegree;
+        row[q] = d > 0;
+        if (mine[q] && gl < d) h.load(v[q], st.cols[b + gl], b + gl, &lab[q], &f[q]);
       }
     }
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-      const double os = __shfl_xor_sync(kFullMask, bs, o);
-      const int32_t ol = __shfl_xor_sync(kFullMask, bl, o);
-      if (ol >= 0 && (bl < 0 || os > bs || (os == bs && ol > bl))) {
-        bs = os;
-        bl = ol;
+    for (int q = 0; q < 2; ++q) {
+      if (!__any_sync(kFullMask, mine[q])) continue;
+      double s = 0.0;
+      bool lead = lab[q] != -1;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) { /* entry order; the first holder leads */
+        const int32_t ol = __shfl_sync(kFullMask, lab[q], k, 8);
+        const double of = __shfl_sync(kFullMask, f[q], k, 8);
+        if (ol == lab[q]) {
+          s += of;
+          if (k < gl) lead = false;
+        }
+      }
+      Scored best{-INFINITY, -1};
+      if (lead) take_better(best, h.score(v[q], lab[q], s), lab[q]);
+      best = group_best<8>(best);
+      if (mine[q] && gl == 0) {
+        if (!row[q]) best.l = st.L[v[q]]; /* isolated: keeps its label */
+        settle(v[q], best);
       }
     }
-    if (lane == 0) {
-      st.Lnext[v] = bl;
-      h.update(v, bl, bs);
-      if (bl != st.L[v]) atomicAdd(changed, 1ull);
-    }
-    __syncwarp();
   }
+
+  nchanged = __reduce_add_sync(kFullMask, nchanged);
+  if (lane == 0 && nchanged) atomicAdd(changed, (unsigned long long)nchanged);
+  if (full) atomicOr(err, kErrProbe);
+}
+
+/* Blocks of k_prop for n vertices on `sms` multiprocessors: four resident
+ * blocks each, fewer when a warp would have no vertex. */
+inline unsigned prop_grid(int32_t n, int32_t sms) {
+  const int64_t want = ((int64_t)n + kPropWarps - 1) / kPropWarps, most = 4ll * (sms > 0 ? sms : 1);
+  return (unsigned)(want < most ? want : most);
 }
 
 /* Launches one iteration (pick, then the propagation step) on `stream`. */
@@ -201,10 +415,7 @@ inline cudaError_t launch_iteration(const H& h, const State& st, const glp_devic
                                     cudaStream_t stream) {
   if (st.n == 0) return cudaSuccess;
   k_pick<H><<<(unsigned)((st.n + 255) / 256), 256, 0, stream>>>(h, st.n);
-  unsigned grid = (unsigned)((st.n + 3) / 4);
-  const unsigned cap = (unsigned)(vw.sms > 0 ? vw.sms : 1) * 64u;
-  if (grid > cap) grid = cap;
-  k_prop<H><<<grid, 128, 0, stream>>>(h, st, vw.hook_keys, vw.hook_vals, vw.changed + iter, vw.err);
+  k_prop<H><<<prop_grid(st.n, vw.sms), kPropThreads, 0, stream>>>(h, st, vw.hook_keys, vw.hook_vals, vw.changed + iter, vw.err);
   return cudaGetLastError();
 }
 
