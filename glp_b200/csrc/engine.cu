@@ -1346,9 +1346,9 @@ static int hooks_iterations(RunCtx& c, H h, int32_t niter, int32_t step0, bool l
       h.st.vol_w = *vol_w;
     }
     glp_hooks::k_pick<H><<<(unsigned)cdiv(g->n, 256), 256, 0, c.s>>>(h, g->n);
-    glp_hooks::k_prop<H><<<glp_hooks::prop_grid(g->n, device_sms()), glp_hooks::kPropThreads, 0, c.s>>>(
-        h, h.st, g->d_hook_keys, g->d_hook_vals, g->d_changed + step, g->d_err);
-    c.launches += 2;
+    GLP_CUDA(glp_hooks::launch_prop(h, h.st, g->max_degree, device_sms(), g->d_hook_keys, g->d_hook_vals,
+                                    g->d_changed + step, g->d_err, c.s));
+    c.launches += g->max_degree > glp_hooks::kBlockDegree ? 3 : 2;
     GLP_CUDA(cudaGetLastError());
     if ((rc = after_iter(c, step, h.st.Lnext))) return rc;
   }

@@ -79,14 +79,41 @@ constexpr uint32_t kFullMask = 0xffffffffu;
 constexpr int kSmemCap = 512; /* runs on graphs with a degree above kSmemCap/2 have the spill tables */
 constexpr uint32_t kErrProbe = 1u;
 
-constexpr int kPropThreads = 256;                 /* k_prop's block size */
+constexpr int kPropThreads = 256;     /* k_prop's block size */
 constexpr int kPropWarps = kPropThreads / 32;
-constexpr int kGroupDegree = 8;                   /* eight lanes per vertex up to here */
-constexpr int kWarpDegree = 128;                  /* a warp per vertex up to here; above, a block */
-constexpr int kBlockSlots = 2048;                 /* block table in shared memory (degree <= 1024) */
-constexpr int kWarpSlots = kBlockSlots / kPropWarps; /* = 2 * kWarpDegree */
-constexpr int kTurnSlots = 512;                   /* buckets that order the warps' adds */
-static_assert(kWarpSlots >= 2 * kWarpDegree && 2 * kWarpDegree <= kSmemCap, "table sizes");
+constexpr int kGroupDegree = 8;       /* eight lanes per vertex up to here */
+constexpr int kWarpDegree = 128;      /* a warp per vertex up to here, */
+constexpr int kBlockDegree = 2047;    /* a block of k_prop up to here; above, k_prop_hub */
+constexpr int kWarpSlots = 2 * kWarpDegree;
+constexpr int kHubThreads = 1024;     /* k_prop_hub's block size */
+static_assert(2 * kWarpDegree <= kSmemCap, "rows that may need the spill tables have them");
+
+/* Shared memory of a block that counts one row: a table of Slots labels that
+ * takes new ones until it holds Close of them (a whole round of new labels
+ * then still fits), and Turns buckets, twice, that order the warps' adds (one
+ * bit per warp). */
+template <int NT, int Slots, int Close, int Turns>
+struct RowShared {
+  static constexpr int kThreads = NT, kWarps = NT / 32, kTurnBuckets = Turns;
+  static constexpr uint32_t kSlots = Slots, kClose = Close;
+  static constexpr int kPerWord = 32 / kWarps; /* buckets per word */
+  static_assert(Close + NT <= Slots && (Turns & (Turns - 1)) == 0, "table and bucket sizes");
+  double vals[Slots];
+  double sf[kWarps][32];
+  struct {
+    double s;
+    int32_t l;
+  } red[kWarps];
+  uint32_t keys[Slots];
+  uint32_t turn[2][Turns / kPerWord];
+  int32_t list[NT];
+  int32_t nlist;
+  uint32_t nkeys;
+};
+using BlockRows = RowShared<kPropThreads, 2560, 2048, 2048>;
+using HubRows = RowShared<kHubThreads, 9216, 4608, 8192>;
+static_assert(kBlockDegree < (int)BlockRows::kClose, "k_prop's rows never overflow its table");
+static_assert(kPropWarps * kWarpSlots <= (int)BlockRows::kSlots, "the warps' tables fit the block's");
 
 /* The 32-bit finaliser of MurmurHash3 (Appleby): slot of a key. */
 __device__ __forceinline__ uint32_t slot_hash(uint32_t k) {
@@ -105,12 +132,48 @@ __global__ void __launch_bounds__(256) k_pick(H h, int32_t n) {
 }
 
 /* Claims or finds the slot of `key` (not 0) among cap slots; cap when the
- * table is full. */
-__device__ __forceinline__ uint32_t claim_slot(uint32_t* keys, uint32_t cap, uint32_t key) {
+ * table is full.  *fresh: whether this call claimed it. */
+__device__ __forceinline__ uint32_t claim_slot(uint32_t* keys, uint32_t cap, uint32_t key, bool* fresh = nullptr) {
   uint32_t slot = __umulhi(slot_hash(key), cap);
   for (uint32_t probe = 0; probe < cap; ++probe) {
     const uint32_t prev = atomicCAS(keys + slot, 0u, key);
-    if (prev == 0u || prev == key) return slot;
+    if (prev == 0u || prev == key) {
+      if (fresh) *fresh = prev == 0u;
+      return slot;
+    }
+    if (++slot == cap) slot = 0u;
+  }
+  return cap;
+}
+/* claim_slot in global memory: four slots are read together before a claim,
+ * so that a key a few probes from home costs two round trips. */
+__device__ __forceinline__ uint32_t claim_spill(uint32_t* keys, uint32_t cap, uint32_t key) {
+  uint32_t slot = __umulhi(slot_hash(key), cap);
+  for (uint32_t probe = 0; probe < cap;) {
+    uint32_t at[4], cur[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      at[i] = slot + i < cap ? slot + i : slot + i - cap; /* cap > 4 */
+      cur[i] = __ldcg(keys + at[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (cur[i] == 0u) cur[i] = atomicCAS(keys + at[i], 0u, key);
+      if (cur[i] == 0u || cur[i] == key) return at[i];
+    }
+    probe += 4;
+    slot = at[3] + 1u < cap ? at[3] + 1u : 0u;
+  }
+  return cap;
+}
+/* The slot that holds `key` in a table no thread is adding keys to; cap when
+ * it is not there. */
+__device__ __forceinline__ uint32_t find_slot(const uint32_t* keys, uint32_t cap, uint32_t key) {
+  uint32_t slot = __umulhi(slot_hash(key), cap);
+  for (uint32_t probe = 0; probe < cap; ++probe) {
+    const uint32_t cur = keys[slot];
+    if (cur == key) return slot;
+    if (cur == 0u) return cap;
     if (++slot == cap) slot = 0u;
   }
   return cap;
@@ -145,7 +208,7 @@ __device__ __forceinline__ Scored group_best(Scored b) {
  * most frequent label has entries (one when all differ). */
 __device__ __forceinline__ bool chunk_freq(int32_t lab, double f, double* sf, double* sum) {
   const int lane = threadIdx.x & 31;
-  __syncwarp();
+  __syncwarp(); /* the previous chunk is read no more */
   sf[lane] = f;
   uint32_t m = __match_any_sync(kFullMask, (uint32_t)lab);
   __syncwarp();
@@ -157,9 +220,142 @@ __device__ __forceinline__ bool chunk_freq(int32_t lab, double f, double* sf, do
   return lead;
 }
 
-/* One propagation step.  A step reads each neighbour's label (and whatever
- * LoadNeighbor asks for) at random, so it is bound by the latency of those
- * reads and by the ordered FP64 sums; the split keeps every warp loading:
+/* Counts row v in the block's table and returns its best label on thread 0.
+ * One chunk of 32 entries per warp at a time: every warp sums its chunk, then
+ * the adds to a label's frequency go in chunk order -- each leader notes its
+ * warp in the turn bucket of its slot and adds after as many barriers as
+ * lower warps share the bucket (none when the labels differ).  The value a
+ * leader adds to is read before the first of these barriers, which the first
+ * in turn may use as it is.  Labels go to the shared table until it closes
+ * (decided between rounds, alike for the whole block); a label that is not
+ * there by then goes to the row's own spill region, entries
+ * [2*off[v], 2*off[v+1]) of gkeys/gvals.  A row's frequent labels come early,
+ * so a hot label's serial adds stay in shared memory and the spill table sees
+ * the rare ones.  sh.turn is all zero at entry and at exit. */
+template <class H, class Sh>
+__device__ __forceinline__ Scored count_row(const H& hook, const State& st, int32_t v, Sh& sh, uint32_t* gkeys,
+                                            double* gvals, int& par, bool& full) {
+  constexpr int NT = Sh::kThreads;
+  H h = hook;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int32_t b = st.off[v];
+  const uint32_t d = (uint32_t)(st.off[v + 1] - b), gcap = 2u * d;
+  const uint32_t cap = gcap < Sh::kSlots ? gcap : Sh::kSlots;
+  uint32_t* keys2 = gkeys + 2ll * b;
+  double* vals2 = gvals + 2ll * b;
+  for (uint32_t s = threadIdx.x; s < cap; s += NT) {
+    sh.keys[s] = 0u;
+    sh.vals[s] = 0.0;
+  }
+  if (d >= Sh::kClose)
+    for (uint32_t s = threadIdx.x; s < gcap; s += NT) {
+      keys2[s] = 0u;
+      vals2[s] = 0.0;
+    }
+  if (threadIdx.x == 0) sh.nkeys = 0u;
+  bool open = true;
+  __syncthreads();
+  for (uint32_t i0 = 0; i0 < d; i0 += 4 * NT) {
+    int32_t lab[4];
+    double f[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t i = i0 + q * NT + threadIdx.x;
+      lab[q] = -1;
+      f[q] = 0.0;
+      if (i < d) h.load(v, st.cols[b + i], b + (int64_t)i, &lab[q], &f[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (d - i0 <= q * NT) break; /* block-uniform */
+      double s, old = 0.0;
+      const bool lead = chunk_freq(lab[q], f[q], sh.sf[warp], &s);
+      double* at = nullptr;
+      uint32_t* turn = nullptr;
+      uint32_t shift = 0;
+      if (lead) {
+        const uint32_t key = (uint32_t)lab[q] + 1u;
+        bool fresh = false;
+        uint32_t slot = open ? claim_slot(sh.keys, cap, key, &fresh) : find_slot(sh.keys, cap, key);
+        if (fresh && d >= Sh::kClose) atomicAdd(&sh.nkeys, 1u);
+        if (slot < cap) at = sh.vals + slot;
+        else if (!open && (slot = claim_spill(keys2, gcap, key)) < gcap) at = vals2 + slot;
+        else full = true;
+        if (at) {
+          const uint32_t bucket = slot & (Sh::kTurnBuckets - 1);
+          turn = &sh.turn[par][bucket / Sh::kPerWord];
+          shift = (bucket % Sh::kPerWord) * Sh::kWarps;
+          atomicOr(turn, 1u << (shift + warp));
+          old = *at;
+        }
+      }
+      __syncthreads();
+      const int rank = at ? __popc((*turn >> shift) & ((1u << warp) - 1u)) : -1;
+      if (d >= Sh::kClose) open = sh.nkeys < Sh::kClose; /* no claim before the next barrier */
+      if (rank == 0) *at = old + s;
+      for (int r = 1; __syncthreads_or(rank >= r); ++r)
+        if (rank == r) *at += s;
+      if (at) *turn = 0u; /* the next round uses the other buckets */
+      par ^= 1;
+    }
+  }
+  Scored best{-INFINITY, -1};
+  for (uint32_t s = threadIdx.x; s < cap; s += NT) {
+    const uint32_t key = sh.keys[s];
+    if (key) take_better(best, h.score(v, (int32_t)(key - 1u), sh.vals[s]), (int32_t)(key - 1u));
+  }
+  if (!open)
+    for (uint32_t s = threadIdx.x; s < gcap; s += NT) {
+      const uint32_t key = keys2[s];
+      if (key) take_better(best, h.score(v, (int32_t)(key - 1u), vals2[s]), (int32_t)(key - 1u));
+    }
+  best = group_best<32>(best);
+  if (lane == 0) {
+    sh.red[warp].s = best.s;
+    sh.red[warp].l = best.l;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < Sh::kWarps; ++w) take_better(best, sh.red[w].s, sh.red[w].l);
+  return best;
+}
+
+/* Counts the block's rows of degree lo..hi: vertices blockIdx.x, blockIdx.x +
+ * gridDim.x, ..., so that the neighbouring large rows of a degree-sorted
+ * graph land on different SMs.  The offsets are scanned a round of NT
+ * vertices at a time (8 bytes a vertex: cheaper than keeping lists in the
+ * public state).  Block-uniform; ends in a barrier. */
+template <class H, class Sh, class Settle>
+__device__ __forceinline__ void count_rows(const H& h, const State& st, int32_t lo, int32_t hi, Sh& sh,
+                                           uint32_t* gkeys, double* gvals, bool& full, const Settle& settle) {
+  constexpr int NT = Sh::kThreads;
+  uint32_t* turn = &sh.turn[0][0];
+  for (uint32_t i = threadIdx.x; i < sizeof(sh.turn) / sizeof(uint32_t); i += NT) turn[i] = 0u;
+  int par = 0;
+  for (int64_t v0 = blockIdx.x; v0 < st.n; v0 += (int64_t)gridDim.x * NT) {
+    if (threadIdx.x == 0) sh.nlist = 0;
+    __syncthreads();
+    const int64_t vt = v0 + (int64_t)threadIdx.x * gridDim.x;
+    if (vt < st.n) {
+      const int32_t d = st.off[vt + 1] - st.off[vt];
+      if (d >= lo && d <= hi) sh.list[atomicAdd(&sh.nlist, 1)] = (int32_t)vt;
+    }
+    __syncthreads();
+    const int32_t nlist = sh.nlist;
+    for (int32_t k = 0; k < nlist; ++k) {
+      const int32_t v = sh.list[k];
+      const Scored best = count_row(h, st, v, sh, gkeys, gvals, par, full);
+      if (threadIdx.x == 0) settle(v, best);
+    }
+    __syncthreads(); /* the list is read no more */
+  }
+  __syncthreads();
+}
+
+/* One propagation step of the rows up to kBlockDegree.  A step reads each
+ * neighbour's label (and whatever LoadNeighbor asks for) at random, so it is
+ * bound by the latency of those reads and by the ordered FP64 sums; the split
+ * keeps every warp loading:
  *   degree 0..8     eight lanes per vertex, four vertices per warp and round,
  *                   two rounds' loads in flight; frequencies by shuffles;
  *   degree 9..32    a warp per vertex, four vertices' entries loaded before
@@ -167,30 +363,15 @@ __device__ __forceinline__ bool chunk_freq(int32_t lab, double f, double* sf, do
  *                   its sums are the final frequencies and need no table;
  *   degree 33..128  a warp per vertex, the whole row loaded first, then a
  *                   per-warp shared table of two slots an entry;
- *   above           a block per vertex, eight chunks at a time: every warp
- *                   sums its chunk, then the adds to a label's frequency go
- *                   in chunk order -- each leader notes its warp in the
- *                   turn bucket of its slot and adds after as many barriers
- *                   as lower warps share the bucket (usually none).  Tables
- *                   in shared memory up to degree 1024, else in the vertex's
- *                   own spill region [2*off[v], 2*off[v+1]) of gkeys/gvals.
- * Vertices are dealt to blocks and warps with the grid as the stride, so
- * that the neighbouring large rows of a degree-sorted graph land on
- * different SMs; every phase scans the offsets for its degrees (8 bytes a
- * vertex, cheaper than keeping lists in the public state).  Measured on one
- * B200, R-MAT scale 20 (31.7 M entries), degree-normalised votes, ten steps:
- * 32 ms; 640 ms with one warp per vertex of any degree, 512 slots cleared and
- * scanned for each and full-warp shuffle sums. */
+ *   to kBlockDegree a block per vertex (count_rows), four blocks to an SM.
+ * Measured on one B200, R-MAT scale 20 (31.4 M entries), degree-normalised
+ * votes, ten steps: 13 ms with k_prop_hub; 640 ms with one warp per
+ * vertex of any degree, 512 slots cleared and scanned for each and full-warp
+ * shuffle sums. */
 template <class H>
-__global__ void __launch_bounds__(kPropThreads, 4) k_prop(H h, const State st, uint32_t* gkeys, double* gvals,
-                                                          unsigned long long* changed, uint32_t* err) {
-  __shared__ double svals[kBlockSlots]; /* the block's table, or one slice per warp */
-  __shared__ uint32_t skeys[kBlockSlots];
-  __shared__ uint32_t sturn[2][kTurnSlots];
-  __shared__ double sf[kPropWarps][32];
-  __shared__ Scored sred[kPropWarps];
-  __shared__ int32_t slist[kPropThreads];
-  __shared__ int32_t sn;
+__global__ void __launch_bounds__(kPropThreads, 4) k_prop(H h, const State st, unsigned long long* changed,
+                                                          uint32_t* err) {
+  __shared__ BlockRows sh;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t nb = gridDim.x, nw = nb * kPropWarps;
   uint32_t nchanged = 0; /* this thread's */
@@ -200,84 +381,11 @@ __global__ void __launch_bounds__(kPropThreads, 4) k_prop(H h, const State st, u
     h.update(v, b.l, b.s);
     nchanged += b.l != st.L[v] ? 1u : 0u;
   };
-
-  /* above kWarpDegree: a block per vertex */
-  for (int i = threadIdx.x; i < 2 * kTurnSlots; i += kPropThreads) (&sturn[0][0])[i] = 0u;
-  int par = 0;
-  for (int64_t v0 = blockIdx.x; v0 < st.n; v0 += nb * kPropThreads) { /* block-uniform */
-    if (threadIdx.x == 0) sn = 0;
-    __syncthreads();
-    const int64_t vt = v0 + threadIdx.x * nb;
-    if (vt < st.n && st.off[vt + 1] - st.off[vt] > kWarpDegree) slist[atomicAdd(&sn, 1)] = (int32_t)vt;
-    __syncthreads();
-    const int32_t nlist = sn;
-    for (int32_t k = 0; k < nlist; ++k) {
-      const int32_t v = slist[k];
-      const int32_t b = st.off[v];
-      const uint32_t d = (uint32_t)(st.off[v + 1] - b), cap = 2u * d;
-      const bool spill = cap > (uint32_t)kBlockSlots;
-      uint32_t* keys = spill ? gkeys + 2ll * b : skeys;
-      double* vals = spill ? gvals + 2ll * b : svals;
-      for (uint32_t s = threadIdx.x; s < cap; s += kPropThreads) {
-        keys[s] = 0u;
-        vals[s] = 0.0;
-      }
-      __syncthreads();
-      for (uint32_t i0 = 0; i0 < d; i0 += 4 * kPropThreads) {
-        int32_t lab[4];
-        double f[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t i = i0 + q * kPropThreads + threadIdx.x;
-          lab[q] = -1;
-          f[q] = 0.0;
-          if (i < d) h.load(v, st.cols[b + i], b + (int64_t)i, &lab[q], &f[q]);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (d - i0 <= q * kPropThreads) break; /* block-uniform */
-          double s;
-          const bool lead = chunk_freq(lab[q], f[q], sf[warp], &s);
-          uint32_t slot = cap;
-          if (lead) {
-            slot = claim_slot(keys, cap, (uint32_t)lab[q] + 1u);
-            full = full || slot == cap;
-          }
-          const bool add = slot < cap;
-          uint32_t* turn = &sturn[par][slot & (kTurnSlots - 1)];
-          if (add) atomicOr(turn, 1u << warp);
-          __syncthreads();
-          const int rank = add ? __popc(*turn & ((1u << warp) - 1u)) : -1;
-          for (int r = 0;; ++r) {
-            if (rank == r) vals[slot] += s;
-            if (!__syncthreads_or(rank > r)) break;
-          }
-          if (add) *turn = 0u; /* the next chunk uses the other bucket set */
-          par ^= 1;
-        }
-      }
-      Scored best{-INFINITY, -1};
-      for (uint32_t s = threadIdx.x; s < cap; s += kPropThreads) {
-        const uint32_t key = keys[s];
-        if (key) {
-          const int32_t l = (int32_t)(key - 1u);
-          take_better(best, h.score(v, l, vals[s]), l);
-        }
-      }
-      best = group_best<32>(best);
-      if (lane == 0) sred[warp] = best;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        for (int w = 1; w < kPropWarps; ++w) take_better(best, sred[w].s, sred[w].l);
-        settle(v, best);
-      }
-    }
-    __syncthreads(); /* the list is read no more */
-  }
+  count_rows(h, st, kWarpDegree + 1, kBlockDegree, sh, nullptr, nullptr, full, settle);
 
   /* 9..kWarpDegree: a warp per vertex */
-  uint32_t* wkeys = skeys + warp * kWarpSlots;
-  double* wvals = svals + warp * kWarpSlots;
+  uint32_t* wkeys = sh.keys + warp * kWarpSlots;
+  double* wvals = sh.vals + warp * kWarpSlots;
   for (int64_t v0 = warp * nb + blockIdx.x; v0 < st.n; v0 += 32 * nw) {
     const int64_t vt = v0 + lane * nw;
     int32_t vb = 0, vd = 0;
@@ -304,7 +412,7 @@ __global__ void __launch_bounds__(kPropThreads, 4) k_prop(H h, const State st, u
         if (v[q] < 0) break; /* warp-uniform */
         double s;
         Scored best{-INFINITY, -1};
-        if (chunk_freq(lab[q], f[q], sf[warp], &s)) take_better(best, h.score(v[q], lab[q], s), lab[q]);
+        if (chunk_freq(lab[q], f[q], sh.sf[warp], &s)) take_better(best, h.score(v[q], lab[q], s), lab[q]);
         best = group_best<32>(best);
         if (lane == 0) settle(v[q], best);
       }
@@ -332,7 +440,7 @@ __global__ void __launch_bounds__(kPropThreads, 4) k_prop(H h, const State st, u
       for (int q = 0; q < 4; ++q) {
         if (32 * q >= d) break; /* warp-uniform */
         double s;
-        if (chunk_freq(lab[q], f[q], sf[warp], &s)) { /* its barriers order the chunks' adds */
+        if (chunk_freq(lab[q], f[q], sh.sf[warp], &s)) { /* its barriers order the chunks' adds */
           const uint32_t slot = claim_slot(wkeys, cap, (uint32_t)lab[q] + 1u);
           if (slot < cap) wvals[slot] += s;
           else full = true;
@@ -400,13 +508,65 @@ __global__ void __launch_bounds__(kPropThreads, 4) k_prop(H h, const State st, u
   nchanged = __reduce_add_sync(kFullMask, nchanged);
   if (lane == 0 && nchanged) atomicAdd(changed, (unsigned long long)nchanged);
   if (full) atomicOr(err, kErrProbe);
+  /* launched on top of k_prop_hub: the step ends when both have.  One block
+   * waits for it; the others leave their SM to the blocks still to come. */
+  if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-/* Blocks of k_prop for n vertices on `sms` multiprocessors: four resident
- * blocks each, fewer when a warp would have no vertex. */
+/* The rows above kBlockDegree: a 1024-thread block per vertex.  One block owns
+ * a row because its sums are ordered, so the step waits for the largest row's
+ * serial rounds, which wide blocks keep few.  k_prop is launched on top
+ * (programmatic launch, independent vertices) and fills the SMs as they run
+ * out of large rows. */
+template <class H>
+__global__ void __launch_bounds__(kHubThreads, 1) k_prop_hub(H h, const State st, uint32_t* gkeys, double* gvals,
+                                                             unsigned long long* changed, uint32_t* err) {
+  extern __shared__ __align__(16) unsigned char hub_smem[];
+  HubRows& sh = *reinterpret_cast<HubRows*>(hub_smem);
+  uint32_t nchanged = 0;
+  bool full = false;
+  asm volatile("griddepcontrol.launch_dependents;");
+  count_rows(h, st, kBlockDegree + 1, INT32_MAX, sh, gkeys, gvals, full, [&](int32_t v, const Scored& b) {
+    st.Lnext[v] = b.l;
+    h.update(v, b.l, b.s);
+    nchanged += b.l != st.L[v] ? 1u : 0u;
+  });
+  if (nchanged) atomicAdd(changed, (unsigned long long)nchanged);
+  if (full) atomicOr(err, kErrProbe);
+}
+
+/* Blocks of k_prop for n vertices on `sms` multiprocessors: four are resident
+ * on each, and four times as many share the vertices, so that SMs that
+ * k_prop_hub leaves late take fewer (R-MAT scale 20, a step: 1.9 ms with
+ * resident blocks only); fewer when a warp would have no vertex. */
 inline unsigned prop_grid(int32_t n, int32_t sms) {
-  const int64_t want = ((int64_t)n + kPropWarps - 1) / kPropWarps, most = 4ll * (sms > 0 ? sms : 1);
+  const int64_t want = ((int64_t)n + kPropWarps - 1) / kPropWarps, most = 16ll * (sms > 0 ? sms : 1);
   return (unsigned)(want < most ? want : most);
+}
+
+/* Launches the propagation step of one iteration on `stream`; gkeys/gvals are
+ * needed from a largest degree above kBlockDegree on. */
+template <class H>
+inline cudaError_t launch_prop(const H& h, const State& st, int32_t max_degree, int32_t sms, uint32_t* gkeys,
+                               double* gvals, unsigned long long* changed, uint32_t* err, cudaStream_t stream) {
+  cudaLaunchAttribute attr = {};
+  cudaLaunchConfig_t cfg = {};
+  if (max_degree > kBlockDegree) {
+    const cudaError_t e = cudaFuncSetAttribute(k_prop_hub<H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(HubRows));
+    if (e != cudaSuccess) return e;
+    k_prop_hub<H><<<(unsigned)(sms > 0 ? sms : 1), kHubThreads, sizeof(HubRows), stream>>>(h, st, gkeys, gvals,
+                                                                                          changed, err);
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+  }
+  cfg.gridDim = dim3(prop_grid(st.n, sms));
+  cfg.blockDim = dim3(kPropThreads);
+  cfg.stream = stream;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_prop<H>, h, st, changed, err);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 /* Launches one iteration (pick, then the propagation step) on `stream`. */
@@ -415,8 +575,7 @@ inline cudaError_t launch_iteration(const H& h, const State& st, const glp_devic
                                     cudaStream_t stream) {
   if (st.n == 0) return cudaSuccess;
   k_pick<H><<<(unsigned)((st.n + 255) / 256), 256, 0, stream>>>(h, st.n);
-  k_prop<H><<<prop_grid(st.n, vw.sms), kPropThreads, 0, stream>>>(h, st, vw.hook_keys, vw.hook_vals, vw.changed + iter, vw.err);
-  return cudaGetLastError();
+  return launch_prop(h, st, vw.max_degree, vw.sms, vw.hook_keys, vw.hook_vals, vw.changed + iter, vw.err, stream);
 }
 
 /* Runs niter iterations of the hook set that make(state) returns, on the

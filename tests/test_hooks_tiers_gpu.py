@@ -32,16 +32,19 @@ def _restate(off, cols, w, lab):
 def _hot_rows():
     """Rows of every class whose neighbours carry two labels after a step:
     many lanes and many warps add to one label's frequency."""
-    degs = [8, 9, 32, 33, 128, 129, 300, 1024, 1025, 2500]
+    degs = [8, 9, 32, 33, 128, 129, 300, 1279, 1280, 2047, 2048, 2500]
     leaves = max(degs)
     edges = [(c, len(degs) + i) for c, d in enumerate(degs) for i in range(d)]
     return undirected(len(degs) + leaves, edges)
 
 
 CASES = {
-    "ladder": lambda: degree_ladder([1, 7, 8, 9, 31, 32, 33, 127, 128, 129, 255, 256, 257, 1023, 1024, 1025, 2047, 2048]),
+    "ladder": lambda: degree_ladder([1, 7, 8, 9, 31, 32, 33, 127, 128, 129, 255, 256, 257, 1279, 1280, 1281, 2047, 2048, 2049]),
     "hot": _hot_rows,
     "star": lambda: star(1500),
+    # the hub rows' shared table closes at 4608 labels: at its edge and beyond it
+    "hub_open": lambda: degree_ladder([4607, 4608, 4609, 6143, 6144, 6145]),
+    "hub_spill": lambda: degree_ladder([7000, 9217, 20000]),
     "tiny": lambda: undirected(3, [(0, 1)]),
 }
 
