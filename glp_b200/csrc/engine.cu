@@ -498,7 +498,9 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     k_hub_scatter<kHubNT, W><<<grid, kHubNT, 2 * sm_hist, L.aux[0]>>>(a, p.hub, p.n_chunks);
     k_hub_bucket<kBucketNT, W, S><<<(unsigned)std::min<int64_t>(p.hub.nitems, device_sms() * 8), kBucketNT, sm, L.aux[0]>>>(
         a, p.hub, score);
-    k_hub_finalize<<<hgrid, 256, 0, L.aux[0]>>>(a, p.hub);
+    const uint8_t* seeds = nullptr;
+    if constexpr (S::kKeep) seeds = score.seeds;
+    k_hub_finalize<<<hgrid, 256, 0, L.aux[0]>>>(a, p.hub, seeds);
     *launches += 6;
     if ((rc = mark_on(L.aux[0], 5, 1))) return rc;
   }
@@ -509,24 +511,28 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     if ((rc = mark_on(s, 7, 1))) return rc;
     ++*launches;
   }
-  if (p.big.n && L.backend != GLP_BACKEND_EXACT) {
-    // a summary screen decides what it can over the whole tier (its work
-    // lists included); the exact kernel takes the vertices it lists
-    if ((rc = mark_on(s, 4, 0))) return rc;
-    GLP_CUDA(cudaMemsetAsync(p.fscreen.count, 0, sizeof(uint32_t), s));
-    TierWork all = work(p.big, 4, &p.fbig);
-    if (L.backend == GLP_BACKEND_CM) {
-      k_big_cm<kBigNT, W, S><<<(unsigned)std::min<int64_t>(p.big.n, kMaxGrid), kBigNT, 0, s>>>(a, all, score,
-                                                                                              p.fscreen);
-    } else {
-      constexpr int kFaNT = 128;
-      k_big_fa<kFaNT, W, S><<<(unsigned)std::min<int64_t>(cdiv(p.big.n, kFaNT / 32), kMaxGrid), kFaNT, 0, s>>>(
-          a, all, score, p.fscreen);
+  bool screened = false;
+  if constexpr (!S::kKeep) screened = p.big.n && L.backend != GLP_BACKEND_EXACT;
+  if (screened) {
+    if constexpr (!S::kKeep) {
+      // a summary screen decides what it can over the whole tier (its work
+      // lists included); the exact kernel takes the vertices it lists
+      if ((rc = mark_on(s, 4, 0))) return rc;
+      GLP_CUDA(cudaMemsetAsync(p.fscreen.count, 0, sizeof(uint32_t), s));
+      TierWork all = work(p.big, 4, &p.fbig);
+      if (L.backend == GLP_BACKEND_CM) {
+        k_big_cm<kBigNT, W, S><<<(unsigned)std::min<int64_t>(p.big.n, kMaxGrid), kBigNT, 0, s>>>(a, all, score,
+                                                                                                p.fscreen);
+      } else {
+        constexpr int kFaNT = 128;
+        k_big_fa<kFaNT, W, S><<<(unsigned)std::min<int64_t>(cdiv(p.big.n, kFaNT / 32), kMaxGrid), kFaNT, 0, s>>>(
+            a, all, score, p.fscreen);
+      }
+      TierWork rest{Verts{nullptr, 0, 0}, p.fscreen, FailList{nullptr, nullptr}, 0, 1};
+      if ((rc = launch_big_list<W, S>(p, a, rest, score, s, launches))) return rc;
+      ++*launches;
+      if ((rc = mark_on(s, 4, 1))) return rc;
     }
-    TierWork rest{Verts{nullptr, 0, 0}, p.fscreen, FailList{nullptr, nullptr}, 0, 1};
-    if ((rc = launch_big_list<W, S>(p, a, rest, score, s, launches))) return rc;
-    ++*launches;
-    if ((rc = mark_on(s, 4, 1))) return rc;
   } else if (p.big.n) {
     // full mode: one launch per degree range, each with the table and block
     // size it needs; outside full mode the tier's majority / frontier list
@@ -550,7 +556,7 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
       if (k16 && r < kBigParts - 1) {
         const size_t sm16 = 12ull * kBigPartMax[r];  // 2*max slots of 4 + 2 bytes
         bool staged = false;
-        if constexpr (S::kPacked) {
+        if constexpr (S::kPacked && !S::kKeep) {
           if (r == 0 && L.big_staged && kBigPartMax[0] <= kStagedRow) {
             // rows staged in shared memory by bulk copies, one vertex ahead
             k_big_staged<256, S><<<grid, 256, sm16, s>>>(a, tw, score);
@@ -586,8 +592,10 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
       }
       ++*launches;
     }
-    if (modal) {
-      if ((rc = launch_big_list<W, S>(p, a, work(Verts{nullptr, 0, 0}, 4, &p.fbig), score, s, launches))) return rc;
+    if constexpr (!S::kKeep) {
+      if (modal &&
+          (rc = launch_big_list<W, S>(p, a, work(Verts{nullptr, 0, 0}, 4, &p.fbig), score, s, launches)))
+        return rc;
     }
     if ((rc = mark_on(s, 4, 1))) return rc;
   }
@@ -603,7 +611,7 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     if (!c16w) {
       // the next vertex's first batch in flight while counting: unweighted
       // classic only (the other instantiations would spill at their register caps)
-      if constexpr (S::kMajority && !W) {
+      if constexpr ((S::kMajority || S::kKeep) && !W) {
         if (L.mid_prefetch) k_mid<kMidCap, kMidNT, W, S, true, true><<<grid, kMidNT, 0, s>>>(a, mw, score);
         else k_mid<kMidCap, kMidNT, W, S><<<grid, kMidNT, 0, s>>>(a, mw, score);
       } else {
@@ -1400,20 +1408,15 @@ static int run_seeded(RunCtx& c, int32_t niter) {
     set_error("method 5 needs seeds: call glp_graph_set_seeds first");
     return GLP_EINVAL;
   }
-  if (g->max_degree > kSeedSmem / 2 && !g->d_seed_keys) {
-    GLP_CUDA(dev_alloc(&g->d_seed_keys, sizeof(uint32_t) * 2 * (size_t)g->m));
-    GLP_CUDA(dev_alloc(&g->d_seed_vals, sizeof(uint32_t) * 2 * (size_t)g->m));
-  }
   k_seeded_init<<<(unsigned)cdiv(g->n, 256), 256, 0, c.s>>>(g->d_seeds, g->d_lab[0], g->d_lab[1], g->n);
   ++c.launches;
-  const unsigned grid = (unsigned)std::min<int64_t>(cdiv(g->n, 8), (int64_t)device_sms() * 16);
   int rc;
   for (int32_t it = 0; it < niter; ++it) {
-    k_seeded_step<W><<<grid, 256, 0, c.s>>>(g->d_off, g->d_cols, g->d_w, g->d_seeds, g->d_lab[it & 1],
-                                            g->d_lab[(it + 1) & 1], g->n, g->d_seed_keys, g->d_seed_vals,
-                                            g->d_changed + it, g->d_err);
-    ++c.launches;
-    GLP_CUDA(cudaGetLastError());
+    // the exact-count tiers of method 1, every vertex in every step
+    const StepArgs a{g->d_off, g->d_cols, g->d_w, g->d_lab[it & 1], g->d_lab[it & 1], g->d_lab[(it + 1) & 1],
+                     g->d_changed + it, g->d_err, nullptr, g->n, nullptr, nullptr};
+    StepLaunch L = c.launch();
+    if ((rc = launch_step<W>(L, a, ScoreSeeded{g->d_seeds}, &c.launches))) return rc;
     if ((rc = after_iter(c, it, g->d_lab[(it + 1) & 1]))) return rc;
   }
   return GLP_OK;
@@ -1594,8 +1597,6 @@ void glp_graph_destroy(glp_graph* g) {
   dev_free(g->d_hook_keys);
   dev_free(g->d_hook_vals);
   dev_free(g->d_seeds);
-  dev_free(g->d_seed_keys);
-  dev_free(g->d_seed_vals);
   if (g->h_cycle) cudaFreeHost(g->h_cycle);
   for (cudaEvent_t e : g->cyc_ev)
     if (e) cudaEventDestroy(e);

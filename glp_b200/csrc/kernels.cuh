@@ -198,6 +198,8 @@ struct TierWork {
 // half of the neighbourhood weight is then the unique maximum, so the
 // majority shortcut applies.
 struct ScoreClassic {
+  static constexpr bool kKeep = false;  // ScoreSeeded: unlabelled neighbours, fixed vertices
+  __device__ __forceinline__ bool fixed(int32_t) const { return false; }
   static constexpr bool kMajority = true;
   // (count << 32 | label) orders candidates as better() does: a block can
   // reduce with one 64-bit shared atomicMax
@@ -227,6 +229,8 @@ struct ScoreClassic {
 // score(l, k) for layered LP: dstar*k - vol_r[l] (kernel.cuh:2575-2600).
 // The volume term breaks the majority argument: no shortcut.
 struct ScoreLayered {
+  static constexpr bool kKeep = false;
+  __device__ __forceinline__ bool fixed(int32_t) const { return false; }
   static constexpr bool kMajority = false;
   static constexpr bool kPacked = false;  // signed 64-bit scores: block_max
   // the volume is a global lookup per label: prefetched per insert, or (step
@@ -261,6 +265,8 @@ struct ScoreLayered {
 // that label) as one 8-byte pair from lv, which the step before wrote
 // (k_label_volumes): one random gather per entry instead of two.
 struct ScoreLayered32 {
+  static constexpr bool kKeep = false;
+  __device__ __forceinline__ bool fixed(int32_t) const { return false; }
   static constexpr bool kMajority = false;
   static constexpr bool kPacked = true;
   static constexpr bool kScan = true;
@@ -285,6 +291,27 @@ struct ScoreLayered32 {
   }
   __device__ __forceinline__ uint32_t key32(uint32_t k, int32_t v) const {
     return (uint32_t)(dstar * (int32_t)k - v) ^ 0x80000000u;
+  }
+};
+
+// Seeded LP (method 5; seeded.cuh): classic counts over the labelled
+// neighbours only (a label of -1 is no entry), seeds fixed, and a vertex
+// without a labelled neighbour keeps its label.  The packed key is count + 1,
+// so that a row with no candidate (key 0) differs from a label of weight 0.
+struct ScoreSeeded {
+  static constexpr bool kKeep = true;
+  static constexpr bool kMajority = false;  // no pre-pass, no frontier: the step is not modal
+  static constexpr bool kPacked = true;
+  static constexpr bool kScan = false;
+  static constexpr int kSMThreads = 2048;
+  static constexpr bool kLV = false;
+  const uint8_t* seeds;
+  __device__ __forceinline__ bool fixed(int32_t v) const { return seeds[v] != 0; }
+  __device__ __forceinline__ int32_t vol_of(int32_t) const { return 0; }
+  __device__ __forceinline__ int64_t from_vol(uint32_t k, int32_t) const { return (int64_t)k; }
+  __device__ __forceinline__ uint32_t key32(uint32_t k, int32_t) const { return k + 1u; }
+  __device__ __forceinline__ void load(const StepArgs& a, int32_t c, int32_t& lab, int32_t&) const {
+    lab = ld_label(a.lin + c);
   }
 };
 
@@ -316,8 +343,10 @@ __global__ void __launch_bounds__(256, TMAX >= 32 ? 2 : 1) k_tiny(StepArgs a, Ti
   const int32_t t = t0 + threadIdx.x;
   bool chg = false;
   int32_t v = 0;
-  if (t < nwork) {
-    v = tw.at(mode, t);
+  if (t < nwork) v = tw.at(mode, t);
+  if (S::kKeep && t < nwork && score.fixed(v)) {
+    a.lout[v] = a.lcur[v];
+  } else if (t < nwork) {
     const int32_t b = a.off[v];
     const int32_t d = a.off[v + 1] - b;
     int32_t lab[TMAX];
@@ -327,6 +356,7 @@ __global__ void __launch_bounds__(256, TMAX >= 32 ? 2 : 1) k_tiny(StepArgs a, Ti
       lab[i] = INT32_MAX;  // past the degree: sorts last, never scored
       wt[i] = 0;
       if (i < d) load_edge<W>(a, (int64_t)b + i, lab[i], wt[i]);
+      if (S::kKeep && lab[i] < 0) lab[i] = INT32_MAX;  // unlabelled: no entry
     }
     sort_labels<TMAX, W>(lab, wt);
     // a run's total is scored at its last element.  Layered LP needs the
@@ -356,8 +386,10 @@ __global__ void __launch_bounds__(256, TMAX >= 32 ? 2 : 1) k_tiny(StepArgs a, Ti
         }
       }
     }
+    const int32_t cur = a.lcur[v];
+    if (S::kKeep && best.l < 0) best.l = cur;
     a.lout[v] = best.l;
-    chg = best.l != a.lcur[v];
+    chg = best.l != cur;
   }
   record_changes(a, chg, v);
   }
@@ -598,7 +630,7 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
   // third full-count step of R-MAT s24, whose labels have begun to gather,
   // 1.12 -> 1.00 ms, the first two unchanged); the layered score does not
   // (measured slower)
-  const bool merge = !CF || mode != kModeFull || S::kMajority;
+  const bool merge = !CF || mode != kModeFull || S::kMajority || S::kKeep;
   uint32_t* kk = skeys[warp];
   uint32_t* vv = svals[warp];
   // batch loader: columns (and weights) of entries j0 + 32q + lane below e,
@@ -648,6 +680,10 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
       b = a.off[v];
       e = a.off[v + 1];
     }
+    if (S::kKeep && score.fixed(v)) {  // warp-uniform
+      if (lane == 0) a.lout[v] = a.lcur[v];
+      continue;
+    }
     // four slots a neighbour where the warp's table holds them, else two: a
     // quarter-full table probes less (measured: rows of degree 33..128 8.2 ->
     // 7.3 ps per entry); degree > 32: cap >= 128
@@ -687,7 +723,9 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
     }
     int32_t lbest;
     if constexpr (S::kPacked) {
-      lbest = (int32_t)(uint32_t)warp_best(best);
+      const unsigned long long wb = warp_best(best);
+      lbest = (int32_t)(uint32_t)wb;
+      if (S::kKeep && !wb) lbest = a.lcur[v];
     } else {
       best = group_max<32>(best);
       lbest = best.l;
@@ -762,6 +800,10 @@ __global__ void __launch_bounds__(NT, (!W ? ((NT == 1024 && S::kPacked) ? 2048 :
     // the vertex's own label, loaded here so that thread 0 does not wait for
     // it after the reduction barrier while the block waits for thread 0
     const int32_t cur = a.lcur[v];
+    if (S::kKeep && score.fixed(v)) {  // block-uniform
+      if (threadIdx.x == 0) a.lout[v] = cur;
+      continue;
+    }
     if (S::kMajority && mode == kModeFrontier) {
       // a frontier vertex of this tier has many neighbours and usually keeps
       // its label: a strict majority of its own label decides it without a
@@ -854,7 +896,7 @@ __global__ void __launch_bounds__(NT, (!W ? ((NT == 1024 && S::kPacked) ? 2048 :
     // on the largest rows, where one label (a hub's own id, carried by its
     // degree-1 neighbours) fills many lanes of a chunk: without it those
     // lanes' adds to one slot serialise
-    const bool merge = !CF || mode != kModeFull || (e - b) > kMergeDegree;
+    const bool merge = !CF || mode != kModeFull || (e - b) > kMergeDegree || S::kKeep;
     for (int32_t j0 = b + warp * 32; j0 < e; j0 += 4 * NT) {
       int32_t lab[4], vl[4];
       uint32_t wt[4];
@@ -883,7 +925,10 @@ __global__ void __launch_bounds__(NT, (!W ? ((NT == 1024 && S::kPacked) ? 2048 :
       const unsigned long long wb = warp_best(best);
       if (lane == 0 && wb) atomicMax(&sbest[par], wb);
       __syncthreads();
-      if (threadIdx.x == 0) lbest = (int32_t)(uint32_t)sbest[par];
+      if (threadIdx.x == 0) {
+        lbest = (int32_t)(uint32_t)sbest[par];
+        if (S::kKeep && !sbest[par]) lbest = cur;
+      }
       par ^= 1;
     } else {
       lbest = block_max<NT>(best, red).l;
@@ -1330,15 +1375,18 @@ __global__ void __launch_bounds__(NT) k_hub_bucket(StepArgs a, HubPlan hp, S sco
   }
 }
 
-__global__ void k_hub_finalize(StepArgs a, HubPlan hp) {
+// `seeds` (seeded LP, else nullptr): seeds keep their label, and so does a hub
+// without a labelled neighbour.
+__global__ void k_hub_finalize(StepArgs a, HubPlan hp, const uint8_t* seeds) {
   const int32_t h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= hp.nhubs) return;
   if (hp.hub_state[h]) return;
   const unsigned long long p = hp.hub_best[h];
   hp.hub_best[h] = 0ull;
   const int32_t v = hp.hub_v[h];
-  const int32_t l = p ? (int32_t)(uint32_t)(p & 0xffffffffull) : a.lcur[v];
-  if (!p) atomicOr(a.err, kErrHubPlan);
+  const bool keep = seeds && (!p || seeds[v]);
+  const int32_t l = p && !keep ? (int32_t)(uint32_t)(p & 0xffffffffull) : a.lcur[v];
+  if (!p && !keep) atomicOr(a.err, kErrHubPlan);
   a.lout[v] = l;
   if (l != a.lcur[v]) record_change(a, v);
 }
