@@ -69,7 +69,7 @@ int device_sms() {
 // so any stream may use it; dev_free is called only once no stream uses the
 // memory any more.
 static std::once_flag g_pool_once[64];
-static cudaError_t dev_alloc_raw(void** p, size_t bytes) {
+cudaError_t dev_alloc_raw(void** p, size_t bytes) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -89,8 +89,23 @@ template <class T>
 static cudaError_t dev_alloc(T** p, size_t bytes) {
   return dev_alloc_raw(reinterpret_cast<void**>(p), bytes);
 }
-static void dev_free(void* p) {
+void dev_free(void* p) {
   if (p) cudaFreeAsync(p, cudaStreamPerThread);
+}
+
+// Gives what the pool holds beyond its live memory and kPoolIdle back to the
+// driver: called after work whose scratch may be many times what it leaves.
+void dev_pool_trim() {
+  constexpr uint64_t kPoolIdle = 4ull << 30;
+  int dev = 0;
+  cudaMemPool_t pool;
+  uint64_t used = 0, held = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaStreamSynchronize(cudaStreamPerThread) == cudaSuccess &&
+      cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+      held > used + kPoolIdle)
+    cudaMemPoolTrimTo(pool, used + kPoolIdle);
 }
 
 // Waits for every stream a handle's work may be on.
@@ -1536,6 +1551,20 @@ int glp_graph_create(const int32_t* offsets, const int32_t* cols, const int32_t*
   return glp_graph_create_ex(offsets, cols, weights, n, m, on_device, 0u, out);
 }
 
+// The streams and events of a new handle on the current device.
+static int open_handle(glp_graph* g, int32_t n, int64_t m) {
+  g->n = n;
+  g->m = m;
+  GLP_CUDA(cudaGetDevice(&g->device));
+  GLP_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
+  GLP_CUDA(cudaStreamCreateWithFlags(&g->aux[0], cudaStreamNonBlocking));
+  GLP_CUDA(cudaStreamCreateWithFlags(&g->aux[1], cudaStreamNonBlocking));
+  GLP_CUDA(cudaEventCreateWithFlags(&g->fork, cudaEventDisableTiming));
+  GLP_CUDA(cudaEventCreateWithFlags(&g->join[0], cudaEventDisableTiming));
+  GLP_CUDA(cudaEventCreateWithFlags(&g->join[1], cudaEventDisableTiming));
+  return GLP_OK;
+}
+
 int glp_graph_create_ex(const int32_t* offsets, const int32_t* cols, const int32_t* weights, int32_t n, int64_t m,
                         int32_t on_device, uint32_t flags, glp_graph** out) {
   if (!out) {
@@ -1550,16 +1579,8 @@ int glp_graph_create_ex(const int32_t* offsets, const int32_t* cols, const int32
   int rc = require_device();
   if (rc) return rc;
   std::unique_ptr<glp_graph> g(new glp_graph());
-  g->n = n;
-  g->m = m;
-  GLP_CUDA(cudaGetDevice(&g->device));
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  GLP_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
-  GLP_CUDA(cudaStreamCreateWithFlags(&g->aux[0], cudaStreamNonBlocking));
-  GLP_CUDA(cudaStreamCreateWithFlags(&g->aux[1], cudaStreamNonBlocking));
-  GLP_CUDA(cudaEventCreateWithFlags(&g->fork, cudaEventDisableTiming));
-  GLP_CUDA(cudaEventCreateWithFlags(&g->join[0], cudaEventDisableTiming));
-  GLP_CUDA(cudaEventCreateWithFlags(&g->join[1], cudaEventDisableTiming));
+  if ((rc = open_handle(g.get(), n, m))) return rc;
   GLP_CUDA(dev_alloc(&g->d_off, sizeof(int32_t) * ((size_t)n + 1)));
   GLP_CUDA(cudaMemcpy(g->d_off, offsets, sizeof(int32_t) * ((size_t)n + 1), kind));
   // 4 padding entries: tile kernels read columns as aligned 16-byte quads
@@ -2123,6 +2144,26 @@ int glp_run_classic_noalloc(const int32_t* d_offsets, const int32_t* d_cols, int
 }  // extern "C"
 
 namespace glp {
+// A handle that takes over a CSR built on the current device: d_off [n+1] and
+// d_cols [m+4], the last four zero, both from dev_alloc_raw, no work on them
+// in flight; rows strictly ascending.  They are freed with the handle, or
+// here on failure.  Not part of the C ABI.
+int graph_adopt(int32_t* d_off, int32_t* d_cols, int32_t n, int64_t m, uint32_t flags, glp_graph** out) {
+  glp_graph* g = new glp_graph();
+  g->d_off = d_off;
+  g->d_cols = d_cols;
+  g->rows_sorted = 1;
+  if (flags & GLP_GRAPH_SYMMETRIC) g->symmetric = 1;
+  int rc = open_handle(g, n, m);
+  if (!rc) rc = validate_csr_device(g);
+  if (rc) {
+    glp_graph_destroy(g);
+    return rc;
+  }
+  *out = g;
+  return GLP_OK;
+}
+
 // Recreates a handle's three streams at `priority` (the order of
 // cudaDeviceGetStreamPriorityRange: lower is more urgent) once its work has
 // finished.  Not part of the C ABI: the server runs short requests at the

@@ -57,6 +57,7 @@ int graph_set_stream_priority(glp_graph* g, int priority);
 int batch_set_stream_priority(glp_batch* b, int priority);
 int ingest_edges(const int32_t* src, const int32_t* dst, int64_t count, int32_t n, int32_t on_device, uint32_t flags,
                  int32_t** d_off, int32_t** d_cols, int64_t* m, int32_t* d_old, cudaStream_t s);
+void dev_pool_trim();
 }  // namespace glp
 
 namespace {
@@ -727,6 +728,7 @@ int glp_server_add_edges(glp_server* s, const int32_t* src, const int32_t* dst, 
   }
   if (old_id && !on_device && d_old) cudaFree(d_old);
   if (st) cudaStreamDestroy(st);
+  glp::dev_pool_trim();
   std::lock_guard<std::mutex> lk(s->mu);
   s->used_bytes -= bound;
   if (rc) {
