@@ -23,7 +23,7 @@
 //                                   test of the own label, else a per-warp
 //                                   shared table;
 //   thread tier (1 <= d <= TT)    : a thread per vertex, labels sorted in
-//                                   registers (bitonic network), counts read
+//                                   registers (sorting network), counts read
 //                                   off the runs.
 // Every step also writes a change flag per vertex (1 byte).  Once few labels
 // still change (fewer than frontier_permille, default 10, per 1000 vertices
@@ -352,7 +352,7 @@ __device__ __forceinline__ bool block_vertex(const BatchArgs& a, int32_t v, cons
 }
 
 // One vertex per thread (1 <= degree <= TT): its labels sorted in registers,
-// counts read off the runs (sort_labels).
+// counts read off the runs (sort_keys).
 template <int TT>
 __device__ __forceinline__ bool thread_vertex(const BatchArgs& a, int32_t v, const int32_t* __restrict__ lin,
                                               int32_t* __restrict__ lout, const uint8_t* __restrict__ fin,
@@ -360,7 +360,6 @@ __device__ __forceinline__ bool thread_vertex(const BatchArgs& a, int32_t v, con
   const int64_t b = a.off[v];
   const int32_t d = (int32_t)(a.off[v + 1] - b);
   int32_t lab[TT];
-  uint32_t one[TT];
 #pragma unroll
   for (int i = 0; i < TT; ++i) lab[i] = i < d ? ld_stream(a.cols + b + i) : -1;
   if (fin) {  // no neighbour changed in the previous step: the label stays
@@ -376,7 +375,7 @@ __device__ __forceinline__ bool thread_vertex(const BatchArgs& a, int32_t v, con
   }
 #pragma unroll
   for (int i = 0; i < TT; ++i) lab[i] = lab[i] >= 0 ? ld_label(lin + lab[i]) : INT32_MAX;
-  sort_labels<TT, false>(lab, one);
+  sort_keys(lab);
   Best best = best_none();
   uint32_t run = 0;
 #pragma unroll

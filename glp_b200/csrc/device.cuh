@@ -56,6 +56,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, uint3
   return false;
 }
 
+// Copies one word to shared memory without passing a register; async_wait
+// waits for this thread's copies.
+__device__ __forceinline__ void async_word(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Dynamic shared memory of the running launch, in bytes.
 __device__ __forceinline__ uint32_t dynamic_smem_bytes() {
   uint32_t r;
@@ -292,38 +299,33 @@ __device__ __forceinline__ void zero_words16(uint32_t* p, uint32_t n, uint32_t t
   for (uint32_t s = t; s < n / 4; s += stride) q[s] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// Sorts TMAX (a power of two) labels held in registers, ascending, with a
-// bitonic network (every index known at compile time, so nothing leaves the
-// registers); weights move with their labels when W.  Equal labels end up
-// adjacent, so a row's counts are the lengths (weight sums) of its runs:
-// O(TMAX log^2 TMAX) min/max steps instead of O(degree * TMAX) compares.
-template <int TMAX, bool W>
-__device__ __forceinline__ void sort_labels(int32_t (&lab)[TMAX], uint32_t (&wt)[TMAX]) {
+// Sorts N keys held in registers, ascending, with Batcher's merge exchange
+// (Knuth, The Art of Computer Programming 3, 5.2.2, algorithm M): every index
+// is known at compile time, so nothing leaves the registers, and N need not be
+// a power of two.  19 / 63 / 97 / 127 / 161 / 191 exchanges for N = 8 / 16 /
+// 20 / 24 / 28 / 32 (a bitonic network: 24 / 80 / 240 for 8 / 16 / 32).
+template <int N, int P, int Q, int R, int D, class K>
+__device__ __forceinline__ void merge_exchange(K (&x)[N]) {
 #pragma unroll
-  for (int k = 2; k <= TMAX; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-#pragma unroll
-      for (int i = 0; i < TMAX; ++i) {
-        const int l = i ^ j;
-        if (l > i) {
-          const bool up = (i & k) == 0;
-          const int32_t x = lab[i], y = lab[l];
-          if (W) {
-            const bool sw = up ? (x > y) : (x < y);
-            const uint32_t wx = wt[i], wy = wt[l];
-            lab[i] = sw ? y : x;
-            lab[l] = sw ? x : y;
-            wt[i] = sw ? wy : wx;
-            wt[l] = sw ? wx : wy;
-          } else {
-            lab[i] = up ? min(x, y) : max(x, y);
-            lab[l] = up ? max(x, y) : min(x, y);
-          }
-        }
-      }
+  for (int i = 0; i < N - D; ++i) {
+    if ((i & P) == R) {
+      const K lo = min(x[i], x[i + D]), hi = max(x[i], x[i + D]);
+      x[i] = lo;
+      x[i + D] = hi;
     }
   }
+  if constexpr (Q != P) {
+    merge_exchange<N, P, Q / 2, P, Q - P>(x);
+  } else if constexpr (P > 1) {
+    constexpr int kTop = N > 16 ? 16 : N > 8 ? 8 : N > 4 ? 4 : N > 2 ? 2 : 1;
+    merge_exchange<N, P / 2, kTop, 0, P / 2>(x);
+  }
+}
+template <int N, class K>
+__device__ __forceinline__ void sort_keys(K (&x)[N]) {
+  static_assert(N >= 2 && N <= 32, "networks of 2..32 keys");
+  constexpr int kTop = N > 16 ? 16 : N > 8 ? 8 : N > 4 ? 4 : N > 2 ? 2 : 1;
+  merge_exchange<N, kTop, kTop, 0, kTop>(x);
 }
 
 // Smallest power of two >= x (x >= 1).

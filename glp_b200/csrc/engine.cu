@@ -453,6 +453,26 @@ static int launch_big_list(const DevicePlan& p, const StepArgs& a, const TierWor
   return GLP_OK;
 }
 
+// One small tier (degree <= R).  Scores with weights or volumes sort label * 32
+// + entry: 32-bit keys while every label (a vertex id) is below 2^27 - 1.
+template <int R, bool W, class S>
+static int launch_small(const StepArgs& a, const TierWork& tw, const S& score, cudaStream_t s) {
+  const unsigned grid = (unsigned)std::min<int64_t>(cdiv(tw.all.n, kSmallNT), device_sms() * 32);
+  const size_t sm = (size_t)(kSmallNT / 32) * small_words<R, W, S>() * sizeof(uint32_t);
+  if constexpr (W || S::kLV) {
+    if (a.n < (1 << 27)) {
+      GLP_CUDA(raise_smem_limit((const void*)k_small<R, W, S, uint32_t>, sm));
+      k_small<R, W, S, uint32_t><<<grid, kSmallNT, sm, s>>>(a, tw, score);
+    } else {
+      GLP_CUDA(raise_smem_limit((const void*)k_small<R, W, S, uint64_t>, sm));
+      k_small<R, W, S, uint64_t><<<grid, kSmallNT, sm, s>>>(a, tw, score);
+    }
+  } else {
+    k_small<R, W, S, int32_t><<<grid, kSmallNT, sm, s>>>(a, tw, score);
+  }
+  return GLP_OK;
+}
+
 template <bool W, class S>
 int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_t* launches) {
   StepLaunch L = Lin;
@@ -638,22 +658,19 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
   }
   if (p.g32.n) {
     if ((rc = mark_on(L.aux[1], 2, 0))) return rc;
-    k_tiny<32, W, S><<<(unsigned)std::min<int64_t>(cdiv(p.g32.n, 256), kMaxGrid), 256, 0, L.aux[1]>>>(
-        a, work(p.g32, 2, nullptr), score);
+    if ((rc = launch_small<32, W>(a, work(p.g32, 2, nullptr), score, L.aux[1]))) return rc;
     if ((rc = mark_on(L.aux[1], 2, 1))) return rc;
     ++*launches;
   }
   if (p.g16.n) {
     if ((rc = mark_on(L.aux[1], 1, 0))) return rc;
-    k_tiny<16, W, S><<<(unsigned)std::min<int64_t>(cdiv(p.g16.n, 256), kMaxGrid), 256, 0, L.aux[1]>>>(
-        a, work(p.g16, 1, nullptr), score);
+    if ((rc = launch_small<16, W>(a, work(p.g16, 1, nullptr), score, L.aux[1]))) return rc;
     if ((rc = mark_on(L.aux[1], 1, 1))) return rc;
     ++*launches;
   }
   if (p.tiny.n) {
     if ((rc = mark_on(L.aux[1], 0, 0))) return rc;
-    k_tiny<8, W, S><<<(unsigned)std::min<int64_t>(cdiv(p.tiny.n, 256), kMaxGrid), 256, 0, L.aux[1]>>>(
-        a, work(p.tiny, 0, nullptr), score);
+    if ((rc = launch_small<8, W>(a, work(p.tiny, 0, nullptr), score, L.aux[1]))) return rc;
     if ((rc = mark_on(L.aux[1], 0, 1))) return rc;
     ++*launches;
   }
@@ -863,29 +880,32 @@ static int ensure_sorted(glp_graph* g) {
 
 // Exact first step when the labels are the vertex ids and rows are strictly
 // ascending: unweighted, the row's last column (k_first_step); weighted, the
-// row's largest (weight, label), per tier: a thread per vertex up to degree
-// 32, a warp per mid vertex, a block per big vertex and hub.
-// Per tier, the neighbour of largest key: a thread per vertex up to degree
-// 32 (eight loads in flight), a warp per mid vertex, a block per big vertex
-// and hub.
+// row's largest (weight, label), per tier (launch_first_keyed).
+// Per tier, the neighbour of largest key: a thread per vertex up to degree 8
+// (eight loads in flight), eight lanes per vertex up to 32 (whole sectors; the
+// planted 2M layer start, weighted, 0.27 -> 0.155 ms; at degree 8 and below
+// they idle: R-MAT s22 0.08 -> 0.13), a warp per mid and big vertex, a block
+// per hub.
 template <class K>
 static int launch_first_keyed(const DevicePlan& p, const StepArgs& a, const K& key, cudaStream_t s,
                               int64_t* launches) {
   const unsigned kMaxGrid = device_sms() * 32;
-  for (const Verts* vs : {&p.tiny, &p.g16, &p.g32})
+  if (p.tiny.n) {
+    k_first_step_w<1, K><<<(unsigned)std::min<int64_t>(cdiv(p.tiny.n, 256), kMaxGrid), 256, 0, s>>>(a, p.tiny, key);
+    ++*launches;
+  }
+  for (const Verts* vs : {&p.g16, &p.g32})
     if (vs->n) {
-      k_first_step_w<1, K><<<(unsigned)std::min<int64_t>(cdiv(vs->n, 256), kMaxGrid), 256, 0, s>>>(a, *vs, key);
+      k_first_step_w<8, K><<<(unsigned)std::min<int64_t>(cdiv((int64_t)vs->n * 8, 256), kMaxGrid), 256, 0, s>>>(a, *vs,
+                                                                                                            key);
       ++*launches;
     }
-  if (p.mid.n) {
-    k_first_step_w<32, K><<<(unsigned)std::min<int64_t>(cdiv((int64_t)p.mid.n * 32, 256), kMaxGrid), 256, 0, s>>>(
-        a, p.mid, key);
-    ++*launches;
-  }
-  if (p.big.n) {
-    k_first_step_w_block<256, K><<<(unsigned)std::min<int64_t>(p.big.n, kMaxGrid), 256, 0, s>>>(a, p.big, key);
-    ++*launches;
-  }
+  for (const Verts* vs : {&p.mid, &p.big})
+    if (vs->n) {
+      k_first_step_w<32, K><<<(unsigned)std::min<int64_t>(cdiv((int64_t)vs->n * 32, 256), kMaxGrid), 256, 0, s>>>(a, *vs,
+                                                                                                              key);
+      ++*launches;
+    }
   if (p.n_hubs) {
     k_first_step_w_block<1024, K><<<(unsigned)p.n_hubs, 1024, 0, s>>>(a, Verts{p.hub.hub_v, 0, p.n_hubs}, key);
     ++*launches;
@@ -1010,6 +1030,8 @@ static int run_classic(RunCtx& c, int32_t niter) {
                g->d_changed + it, g->d_err, p.d_mode, g->n, fr ? p.chg[it & 1] : nullptr,
                fr ? p.counts + 7 + (it & 1) : nullptr};
     a.bb = bb;
+    // the change list's readers: the cycle check and the next step's frontier
+    a.chg_cap = std::max(cyc_cap, (uint32_t)((uint64_t)g->n * c.frontier_pm / 1000) + 1u);
     if (fr) GLP_CUDA(cudaMemsetAsync(p.counts + 7 + (it & 1), 0, sizeof(uint32_t), c.s));
     StepLaunch L = c.launch();
     L.prev_changed = it > 0 ? g->d_changed + it - 1 : nullptr;

@@ -9,8 +9,8 @@
 // label buffers hold their label, so they keep it (kernel.cuh:4387-4390).
 //
 // Tiers (chosen by the host planner from the degree):
-//   tiny  (1..8)       : one thread per vertex, labels in registers
-//   group (9..32)      : 16 or 32 lanes per vertex, one __match_any_sync round
+//   small (1..32)      : one thread per vertex, labels sorted in registers;
+//                        three launches (<= 8, <= 16, <= 32)
 //   mid   (33..256)    : one warp per vertex, per-warp shared-memory table
 //   big   (257..24576) : one block per vertex, block shared-memory table
 //   hub   (above big)  : labels gathered once and sorted into hash buckets,
@@ -62,28 +62,42 @@ struct StepArgs {
   // this step's mode, set on the device by k_step_mode (nullptr: full)
   const int32_t* mode;
   int32_t n;
-  // vertices whose label changed this step are appended here (nullable)
+  // vertices whose label changed this step are appended here (nullable); a
+  // list longer than chg_cap has no reader, so kernels may stop adding to it
   int32_t* chg_out;
   uint32_t* chg_out_n;
   BigBound bb{};
+  uint32_t chg_cap = 0xffffffffu;
 };
 
-// Counts (and, when a.chg_out is set, lists) the vertices whose label changed.
-// Every lane of the warp calls it; v is only read when changed.
-__device__ __forceinline__ void record_changes(const StepArgs& a, bool changed, int32_t v) {
+// Changes of kernels whose warps decide 32 vertices at a time: every lane
+// calls note_changes after its vertex and tally_changes at the end.  The
+// counter takes one add per warp, and the list one reservation per warp and
+// round until one comes back past chg_cap.  (An add to each per warp and round
+// queued 600 thousand atomics on two words when most of 10 M vertices changed:
+// the first step 0.40 -> 0.17 ms.  A block-wide tally behind a barrier cost
+// the small tiers of weighted layered LP 15 %.)
+struct ChangeNotes {
+  uint32_t count = 0;
+  bool listing;
+  __device__ __forceinline__ explicit ChangeNotes(const StepArgs& a) : listing(a.chg_out != nullptr) {}
+};
+__device__ __forceinline__ void note_changes(const StepArgs& a, ChangeNotes& notes, bool changed, int32_t v) {
+  notes.count += changed ? 1u : 0u;
+  if (!notes.listing) return;  // warp-uniform
   const uint32_t m = __ballot_sync(kFull, changed);
   if (!m) return;
   const int lane = threadIdx.x & 31;
   const int leader = __ffs(m) - 1;
   uint32_t base = 0;
-  if (lane == leader) {
-    atomicAdd(a.changed, (unsigned long long)__popc(m));
-    if (a.chg_out) base = atomicAdd(a.chg_out_n, (uint32_t)__popc(m));
-  }
-  if (a.chg_out) {
-    base = __shfl_sync(kFull, base, leader);
-    if (changed) a.chg_out[base + __popc(m & ((1u << lane) - 1u))] = v;
-  }
+  if (lane == leader) base = atomicAdd(a.chg_out_n, (uint32_t)__popc(m));
+  base = __shfl_sync(kFull, base, leader);
+  if (base > a.chg_cap) notes.listing = false;
+  else if (changed) a.chg_out[base + __popc(m & ((1u << lane) - 1u))] = v;
+}
+__device__ __forceinline__ void tally_changes(const StepArgs& a, const ChangeNotes& notes) {
+  const uint32_t c = __reduce_add_sync(kFull, notes.count);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(a.changed, (unsigned long long)c);
 }
 
 // The same for one thread deciding alone.
@@ -333,125 +347,227 @@ __device__ __forceinline__ unsigned long long pack_best(const Best& b, uint32_t*
   return ((unsigned long long)s << 32) | (uint32_t)b.l;
 }
 
-// ---------------------------------------------------------------- tiny tier
-template <int TMAX, bool W, class S>
-__global__ void __launch_bounds__(256, TMAX >= 32 ? 2 : 1) k_tiny(StepArgs a, TierWork tw, S score) {
-  const int32_t mode = step_mode(a);
-  const int32_t nwork = tw.size(mode);
-  // grid-stride over whole warps so record_changes sees full warps
-  for (int32_t t0 = blockIdx.x * blockDim.x; t0 < nwork; t0 += gridDim.x * blockDim.x) {
-  const int32_t t = t0 + threadIdx.x;
-  bool chg = false;
-  int32_t v = 0;
-  if (t < nwork) v = tw.at(mode, t);
-  if (S::kKeep && t < nwork && score.fixed(v)) {
-    a.lout[v] = a.lcur[v];
-  } else if (t < nwork) {
-    const int32_t b = a.off[v];
-    const int32_t d = a.off[v + 1] - b;
-    int32_t lab[TMAX];
-    uint32_t wt[TMAX];
+// -------------------------------------------------------------- small tiers
+// Degree <= R (8, 16 or 32): a warp takes 32 vertices.  Their rows are loaded
+// by eight lanes each, four rows at a time (whole sectors, four or eight loads
+// in flight a lane), and the labels, weights and volumes go to shared memory;
+// then each thread sorts its own vertex's labels in registers and reads the
+// counts off the runs.  The label gather bounds it: at 3.4 ps per entry on
+// planted 10M (degrees 17..32, 170 M entries: 0.57 ms) it runs at the rate at
+// which random 32-byte sectors come from L2 (3.3 ps, measured with the columns
+// streamed and nothing counted).  Before, a thread loaded its own row (32
+// sectors a load instead of about six: the L1 wavefronts bound it) and sorted
+// 32 labels with a bitonic network: 0.73 ms; with weights and a gather per
+// distinct label's volume, weighted layered planted 2M, 0.29 -> 0.25 ms.
+//
+// Entry i of thread t's row sits in word small_at<R>(t, i): eight lanes storing
+// eight entries of four rows, and 32 threads reading entry i of their rows, both
+// touch 32 different banks.
+template <int R>
+__device__ __forceinline__ int small_turn(int t) {
+  constexpr int k = 32 / R;
+  return 8 * ((t / k) % (k < 4 ? 4 / k : 1)) + (t >> 2);
+}
+template <int R>
+__device__ __forceinline__ int small_at(int t, int i) {
+  return t * R + ((i + small_turn<R>(t)) & (R - 1));
+}
+// Words of shared memory per warp: labels, and weights and volumes where the
+// score has them.
+template <int R, bool W, class S>
+constexpr int small_words() {
+  return 32 * R * (1 + (W ? 1 : 0) + (S::kLV ? 1 : 0));
+}
+
+// The best (score, label) of one row, N >= its degree d: the labels are sorted
+// (K: as they are; with weights or volumes to follow, label * 32 + entry), the
+// running total of a run never exceeds its last one, and equal scores come in
+// ascending label order, so the last best element is the answer.  `own`: the
+// thread's first words.
+template <int N, int R, bool W, class S, class K>
+__device__ __forceinline__ int32_t small_best(const StepArgs& a, const S& score, const uint32_t* slab, int t, int d) {
+  constexpr bool kKeyed = W || S::kLV;
+  constexpr K kNone = kKeyed ? (K)~(K)0 : (K)INT32_MAX;
+  const uint32_t* sw = slab + 32 * R;
+  const uint32_t* svol = slab + 32 * R * (W ? 2 : 1);
+  K key[N];
 #pragma unroll
-    for (int i = 0; i < TMAX; ++i) {
-      lab[i] = INT32_MAX;  // past the degree: sorts last, never scored
-      wt[i] = 0;
-      if (i < d) load_edge<W>(a, (int64_t)b + i, lab[i], wt[i]);
-      if (S::kKeep && lab[i] < 0) lab[i] = INT32_MAX;  // unlabelled: no entry
+  for (int i = 0; i < N; ++i) {
+    key[i] = kNone;
+    if (i < d) {
+      const uint32_t l = slab[small_at<R>(t, i)];
+      if (!S::kKeep || (int32_t)l >= 0) key[i] = kKeyed ? (K)((K)l << 5 | (K)i) : (K)l;  // unlabelled: no entry
     }
-    sort_labels<TMAX, W>(lab, wt);
-    // a run's total is scored at its last element.  Layered LP needs the
-    // label's volume there: loaded for run ends only, eight slots a round so
-    // that the loads of a round are in flight together without holding a
-    // register per slot
-    constexpr int U = TMAX < 8 ? TMAX : 8;
-    Best best = best_none();
-    uint32_t run = 0;
+  }
+  sort_keys(key);
+  int32_t bl = -1;
+  std::conditional_t<S::kPacked, uint32_t, int64_t> bs{};
+  uint32_t run = 0;
+  constexpr int U = N < 8 ? N : 8;  // global volume lookups in flight
 #pragma unroll
-    for (int i0 = 0; i0 < TMAX; i0 += U) {
-      int32_t vl[U];
+  for (int i0 = 0; i0 < N; i0 += U) {
+    int32_t vl[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int i = i0 + u;
-        const bool end = (i == TMAX - 1) || lab[(i + 1) & (TMAX - 1)] != lab[i];
-        vl[u] = (S::kScan && end && lab[i] != INT32_MAX) ? score.vol_of(lab[i]) : 0;
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int i = i0 + u;
-        run = (i > 0 && lab[i] == lab[i > 0 ? i - 1 : 0]) ? run + wt[i] : wt[i];
-        const bool end = (i == TMAX - 1) || lab[(i + 1) & (TMAX - 1)] != lab[i];
-        if (end && lab[i] != INT32_MAX) {
-          const Best c{score.from_vol(run, vl[u]), lab[i]};
-          if (better(c, best)) best = c;
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u;
+      if (i >= N) break;
+      const int32_t l = (int32_t)(kKeyed ? key[i] >> 5 : key[i]);
+      vl[u] = 0;
+      if (key[i] != kNone) {
+        const int at = small_at<R>(t, (int)(key[i] & 31));
+        if constexpr (S::kLV) {
+          vl[u] = (int32_t)svol[at];
+        } else if constexpr (S::kScan) {  // a run is scored at its last element only
+          const bool end = i == N - 1 || (kKeyed ? key[i + 1 < N ? i + 1 : i] >> 5 : key[i + 1 < N ? i + 1 : i]) != (K)l;
+          if (end) vl[u] = score.vol_of(l);
         }
       }
     }
-    const int32_t cur = a.lcur[v];
-    if (S::kKeep && best.l < 0) best.l = cur;
-    a.lout[v] = best.l;
-    chg = best.l != cur;
-  }
-  record_changes(a, chg, v);
-  }
-}
-
-// --------------------------------------------------------------- group tier
-// G lanes per vertex (degree <= G); each warp handles U rounds of 32/G
-// vertices with all loads issued before any counting.  The match key carries
-// the group index so equal labels of different vertices do not merge.
-template <int G, int U, bool W, class S>
-__global__ void __launch_bounds__(256) k_group(StepArgs a, TierWork tw, S score) {
-  constexpr int PER = 32 / G;
-  const int32_t mode = step_mode(a);
-  const int32_t nwork = tw.size(mode);
-  const int lane = threadIdx.x & 31;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp * U * PER < nwork;
-       warp += nwarps) {
-  int32_t v[U], lab[U];
-  uint32_t wt[U];
-  bool act[U], has[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const int64_t grp = (warp * U + u) * PER + lane / G;
-    act[u] = grp < nwork;
-    has[u] = false;
-    v[u] = 0;
-    wt[u] = 0;
-    int32_t col = 0;
-    if (act[u]) {
-      v[u] = tw.at(mode, grp);
-      const int32_t b = a.off[v[u]], e = a.off[v[u] + 1];
-      const int32_t j = b + (lane & (G - 1));
-      has[u] = j < e;
-      if (has[u]) {
-        col = ld_stream(a.cols + j);
-        if (W) wt[u] = (uint32_t)ld_stream(a.w + j);
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u;
+      if (i >= N) break;
+      if (key[i] == kNone) continue;
+      const int32_t l = (int32_t)(kKeyed ? key[i] >> 5 : key[i]);
+      const bool same = i > 0 && (kKeyed ? key[i ? i - 1 : 0] >> 5 : key[i ? i - 1 : 0]) == (K)l;
+      const uint32_t w = W ? sw[small_at<R>(t, (int)(key[i] & 31))] : 1u;
+      run = same ? run + w : w;
+      if constexpr (S::kScan && !S::kLV) {
+        const bool end = i == N - 1 || (kKeyed ? key[i + 1 < N ? i + 1 : i] >> 5 : key[i + 1 < N ? i + 1 : i]) != (K)l;
+        if (!end) continue;
+      }
+      if constexpr (S::kPacked) {
+        const uint32_t c = score.key32(run, vl[u]);
+        if (bl < 0 || c >= bs) {
+          bs = c;
+          bl = l;
+        }
+      } else {
+        const int64_t c = score.from_vol(run, vl[u]);
+        if (bl < 0 || c >= bs) {
+          bs = c;
+          bl = l;
+        }
       }
     }
-    lab[u] = col;
   }
-#pragma unroll
-  for (int u = 0; u < U; ++u) lab[u] = has[u] ? ld_label(a.lin + lab[u]) : -1;
-  uint32_t chg = 0;
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const unsigned long long key = ((unsigned long long)(lane / G) << 32) | (uint32_t)lab[u];
-    const uint32_t m = __match_any_sync(kFull, key);
-    const uint32_t k = W ? __reduce_add_sync(m, wt[u]) : (uint32_t)__popc(m);
-    Best c = best_none();
-    if (has[u] && lane == __ffs(m) - 1) c = Best{score(lab[u], k), lab[u]};
-    c = group_max<G>(c);
-    const bool writer = act[u] && (lane & (G - 1)) == 0;
-    bool ch = false;
-    if (writer) {
-      a.lout[v[u]] = c.l;
-      ch = c.l != a.lcur[v[u]];
+  return bl;
+}
+
+// K: uint32_t sort keys (keyed scores: every label below 2^27 - 1), else
+// uint64_t.
+constexpr int kSmallNT = 256;
+// Blocks per SM that the shared memory leaves room for, at most four.
+template <int R, bool W, class S>
+constexpr int small_blocks() {
+  constexpr int n = 221184 / (kSmallNT / 32 * small_words<R, W, S>() * 4 + 1024);
+  return n < 4 ? n : 4;
+}
+template <int R, bool W, class S, class K>
+__global__ void __launch_bounds__(kSmallNT, sizeof(K) == 4 ? small_blocks<R, W, S>() : 2) k_small(StepArgs a, TierWork tw, S score) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t* slab = smem + warp * small_words<R, W, S>();
+  uint32_t* sw = slab + 32 * R;
+  uint32_t* svol = slab + 32 * R * (W ? 2 : 1);
+  const int32_t mode = step_mode(a);
+  const int32_t nwork = tw.size(mode);
+  const int64_t stride = (int64_t)gridDim.x * kSmallNT;
+  ChangeNotes notes(a);
+  for (int64_t t0 = (int64_t)blockIdx.x * kSmallNT + warp * 32; t0 < nwork; t0 += stride) {  // warp-uniform
+    const int64_t tv = t0 + lane;
+    const bool has = tv < nwork;
+    int32_t v = 0, b = 0, d = 0, cur = 0;
+    bool fixed = false;
+    if (has) {
+      v = tw.at(mode, tv);
+      cur = a.lcur[v];
+      fixed = S::kKeep && score.fixed(v);
+      b = a.off[v];
+      d = fixed ? 0 : a.off[v + 1] - b;
     }
-    record_changes(a, ch, v[u]);
+    const int dmax = (int)__reduce_max_sync(kFull, (uint32_t)d);
+    // a lane helps to load rows 4g + lane / 8, eight of them in flight
+    const int grp = lane >> 3;
+    if constexpr (R < 32 || W || S::kLV) {
+      // all columns (and weights) first, which takes no registers, then the
+      // labels; a lane gathers for what it copied.  (Fewer rounds of latency:
+      // weighted layered planted 2M 19.1 -> 17.2 ms; degrees 17..32 with labels
+      // alone have warps enough to hide them and ran 3 % slower so.)
+#pragma unroll 1
+      for (int c0 = 0; c0 < dmax; c0 += 8) {
+        const int i = c0 + (lane & 7);
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const int32_t rb = __shfl_sync(kFull, b, 4 * g + grp), rd = __shfl_sync(kFull, d, 4 * g + grp);
+          if (i < rd) {
+            const int at = small_at<R>(4 * g + grp, i);
+            async_word(slab + at, a.cols + rb + i);
+            if (W) async_word(sw + at, a.w + rb + i);
+          }
+        }
+      }
+      async_wait();
+#pragma unroll 1
+      for (int c0 = 0; c0 < dmax; c0 += 8) {
+        const int i = c0 + (lane & 7);
+        int32_t lab[8], vl[8];
+        bool in[8];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          in[g] = i < __shfl_sync(kFull, d, 4 * g + grp);
+          if (in[g]) score.load(a, (int32_t)slab[small_at<R>(4 * g + grp, i)], lab[g], vl[g]);
+        }
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          if (in[g]) {
+            const int at = small_at<R>(4 * g + grp, i);
+            slab[at] = (uint32_t)lab[g];
+            if (S::kLV) svol[at] = (uint32_t)vl[g];
+          }
+        }
+      }
+    } else {
+#pragma unroll 1
+      for (int c0 = 0; c0 < dmax; c0 += 8) {
+        const int i = c0 + (lane & 7);
+        int32_t lab[8], vl[8];
+        bool in[8];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const int32_t j = __shfl_sync(kFull, b, 4 * g + grp) + i;
+          in[g] = i < __shfl_sync(kFull, d, 4 * g + grp);
+          lab[g] = in[g] ? ld_stream(a.cols + j) : -1;
+        }
+#pragma unroll
+        for (int g = 0; g < 8; ++g)
+          if (in[g]) score.load(a, lab[g], lab[g], vl[g]);
+#pragma unroll
+        for (int g = 0; g < 8; ++g)
+          if (in[g]) slab[small_at<R>(4 * g + grp, i)] = (uint32_t)lab[g];
+      }
+    }
+    __syncwarp();
+    int32_t best = -1;
+    // the network of the warp's largest degree (neighbouring vertices of a
+    // degree-sorted graph have about the same)
+    if (R == 8) {
+      best = dmax <= 4 ? small_best<4, R, W, S, K>(a, score, slab, lane, d) : small_best<8, R, W, S, K>(a, score, slab, lane, d);
+    } else if (R == 16) {
+      best = dmax <= 12 ? small_best<12, R, W, S, K>(a, score, slab, lane, d)
+                        : small_best<16, R, W, S, K>(a, score, slab, lane, d);
+    } else if constexpr (R == 32) {
+      best = dmax <= 20   ? small_best<20, R, W, S, K>(a, score, slab, lane, d)
+             : dmax <= 24 ? small_best<24, R, W, S, K>(a, score, slab, lane, d)
+             : dmax <= 28 ? small_best<28, R, W, S, K>(a, score, slab, lane, d)
+                          : small_best<32, R, W, S, K>(a, score, slab, lane, d);
+    }
+    if (best < 0) best = cur;  // a seed, or no labelled neighbour
+    if (has) a.lout[v] = best;
+    note_changes(a, notes, has && best != cur, v);
+    __syncwarp();  // the words are stored for the next vertices
   }
-  (void)chg;
-  }
+  tally_changes(a, notes);
 }
 
 // Count one 32-edge chunk: every lane adds its own label to the table and
@@ -1446,6 +1562,7 @@ __global__ void k_cycle_verdict(const uint32_t* mism, volatile uint32_t* flag) {
 // the row's last column.  Exact for classic LP and the SLPA listener
 // (unweighted).
 __global__ void __launch_bounds__(256) k_first_step(StepArgs a) {
+  ChangeNotes notes(a);
   for (int32_t v0 = blockIdx.x * blockDim.x; v0 < a.n; v0 += gridDim.x * blockDim.x) {
     const int32_t v = v0 + threadIdx.x;
     bool chg = false;
@@ -1457,14 +1574,15 @@ __global__ void __launch_bounds__(256) k_first_step(StepArgs a) {
         chg = l != a.lcur[v];
       }
     }
-    record_changes(a, chg, v);
+    note_changes(a, notes, chg, v);
   }
+  tally_changes(a, notes);
 }
 
 // The weighted form of the same shortcut: every neighbour label occurs once,
 // so its count is the edge's weight, and the step takes the neighbour label
 // of largest (weight, label).  G lanes per vertex (1 or 32); the rows of the
-// big tier and the hubs go to k_first_step_w_block.  The key of an entry is
+// hubs go to k_first_step_w_block.  The key of an entry is
 // a 64-bit word monotone in (score, label) and never 0 for a candidate.
 struct FirstKeyW {
   __device__ __forceinline__ unsigned long long operator()(const StepArgs& a, int32_t j) const {
@@ -1489,6 +1607,7 @@ struct FirstKeyLayered {
 template <int G, class K = FirstKeyW>
 __global__ void __launch_bounds__(256) k_first_step_w(StepArgs a, Verts vs, K key = K{}) {
   const int lane = threadIdx.x & (G - 1);
+  ChangeNotes notes(a);
   for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x; t0 < (int64_t)vs.n * G; t0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = (t0 + threadIdx.x) / G;
     bool chg = false;
@@ -1505,7 +1624,11 @@ __global__ void __launch_bounds__(256) k_first_step_w(StepArgs a, Verts vs, K ke
             if (j0 + q < e) best = max(best, key(a, j0 + q));
         }
       } else {
-        for (int32_t j = b + lane; j < e; j += G) best = max(best, key(a, j));
+        for (int32_t j0 = b + lane; j0 < e; j0 += 4 * G) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (j0 + q * G < e) best = max(best, key(a, j0 + q * G));
+        }
       }
     }
 #pragma unroll
@@ -1515,8 +1638,9 @@ __global__ void __launch_bounds__(256) k_first_step_w(StepArgs a, Verts vs, K ke
       a.lout[v] = l;
       chg = l != a.lcur[v];
     }
-    record_changes(a, chg, v);
+    note_changes(a, notes, chg, v);
   }
+  tally_changes(a, notes);
 }
 template <int NT, class K = FirstKeyW>
 __global__ void __launch_bounds__(NT) k_first_step_w_block(StepArgs a, Verts vs, K key = K{}) {
@@ -1527,7 +1651,11 @@ __global__ void __launch_bounds__(NT) k_first_step_w_block(StepArgs a, Verts vs,
     if (threadIdx.x == 0) sb = 0ull;
     __syncthreads();
     unsigned long long best = 0ull;
-    for (int32_t j = b + threadIdx.x; j < e; j += NT) best = max(best, key(a, j));
+    for (int32_t j0 = b + threadIdx.x; j0 < e; j0 += 4 * NT) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (j0 + q * NT < e) best = max(best, key(a, j0 + q * NT));
+    }
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) best = max(best, __shfl_xor_sync(kFull, best, m));
     if ((threadIdx.x & 31) == 0) atomicMax(&sb, best);
