@@ -286,6 +286,7 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
   DevicePlan& p = g->plan;
   p.tiers = t;
   p.setup = g->stream;
+  p.sorted = g->deg_sorted == 1;
   // weighted mid counts fit 16 bits when no mid vertex's weights sum past it
   p.mid_c16 = g->d_w == nullptr || g->mid_wsum < 65536u;
   int rc;
@@ -493,14 +494,12 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
                                 L.allow_frontier, L.majority_pm, L.frontier_pm, p.d_mode);
     ++*launches;
     if (L.allow_frontier && L.front.chg_in) {
-      const unsigned fgrid = device_sms() * 16;
-      k_frontier_push<<<fgrid, 256, 0, s>>>(a, L.front);
-      k_frontier_copy<<<fgrid, 256, 0, s>>>(a, L.front);
+      k_frontier_push<<<device_sms() * 16, 256, 0, s>>>(a, L.front);
+      // a degree-sorted graph's isolated vertices come last and are no one's neighbours
+      const int32_t nscan = p.sorted ? a.n - (int32_t)p.isolated : a.n;
+      k_frontier_list<<<(unsigned)std::min<int64_t>(cdiv(a.n, kListRound), device_sms() * 8), 256, 0, s>>>(a, L.front, nscan,
+                                                                                             p.hub);
       *launches += 2;
-      if (p.n_hubs) {
-        k_frontier_hubs<<<(unsigned)cdiv(p.n_hubs, 256), 256, 0, s>>>(a, L.front, p.hub);
-        ++*launches;
-      }
     }
   }
   auto work = [&](const Verts& all, int k, const FailList* major) {

@@ -92,6 +92,7 @@ struct DevicePlan {
   bool mid_c16 = true;  // mid counts fit 16 bits (unweighted, or small weight sums)
   int32_t n_hubs = 0, n_chunks = 0;
   int64_t isolated = 0;
+  bool sorted = false;  // degrees never increase along the ids: every tier is a range, isolated vertices last
   HubPlan hub{};
   BigBound bb{};  // count bounds of a contiguous big tier (n = 0: the tier is an id list)
   std::vector<void*> allocs;

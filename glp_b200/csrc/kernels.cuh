@@ -1707,57 +1707,107 @@ struct Frontier {
   FailList tier[5];        // frontier members of tiny, g16, g32, mid, big
 };
 
-// One warp per changed vertex marks its neighbours; the first marker of a
-// vertex lists it in its tier (hubs are picked up by k_frontier_hubs).
+// Marks the neighbours of the changed vertices (and counts, for the big tier's
+// bounds, each of its members' changed neighbours): eight lanes per changed
+// vertex, a warp for rows above kPushRow.  A mark is a plain store: which
+// vertices are marked is collected afterwards, in id order, by
+// k_frontier_list.  (Listing a vertex when it is first marked took an atomic
+// exchange and two gathers per entry and an add to a tier's counter per warp
+// and entry group: the first frontier step of planted 10M, 0.5 M changed
+// vertices, 0.74 ms; push and list now take 0.12.)
+constexpr int32_t kPushRow = 256;
+__device__ __forceinline__ void push_entry(const StepArgs& a, const Frontier& f, int32_t j) {
+  const int32_t x = ld_stream(a.cols + j);
+  f.act[x] = f.epoch;
+  if (a.bb.has(x)) atomicAdd(a.bb.nchg + (x - a.bb.base), 1u);
+}
 __global__ void __launch_bounds__(256) k_frontier_push(StepArgs a, Frontier f) {
   if (step_mode(a) != kModeFrontier) return;
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const uint32_t nc = *f.chg_in_n;
-  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nc; i += nw) {
-    const int32_t u = f.chg_in[i];
-    const int32_t b = a.off[u], e = a.off[u + 1];
-    for (int32_t j0 = b; j0 < e; j0 += 32) {
-      const int32_t j = j0 + lane;
-      int tier = -1;
-      int32_t x = 0;
-      if (j < e) {
-        x = ld_stream(a.cols + j);
-        if (a.bb.has(x)) atomicAdd(a.bb.nchg + (x - a.bb.base), 1u);
-        if (atomicExch(f.act + x, f.epoch) != f.epoch) {
-          const int32_t d = a.off[x + 1] - a.off[x];
-          tier = d <= f.tiny_max ? 0 : d <= 16 ? 1 : d <= 32 ? 2 : d <= f.mid_max ? 3 : d <= f.big_max ? 4 : -1;
-        }
-      }
+  for (int64_t i0 = 4 * (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); i0 < nc; i0 += 4 * nw) {
+    const int64_t i = i0 + (lane >> 3);
+    int32_t b = 0, d = 0;
+    if (i < nc) {
+      const int32_t u = f.chg_in[i];
+      b = a.off[u];
+      d = a.off[u + 1] - b;
+    }
+    const int32_t dg = d <= kPushRow ? d : 0;
+    for (int32_t c0 = lane & 7; c0 < dg; c0 += 32) {
 #pragma unroll
-      for (int t = 0; t < 5; ++t) {
-        const uint32_t m = __ballot_sync(kFull, tier == t);
-        if (!m) continue;
-        uint32_t base = 0;
-        if (lane == __ffs(m) - 1) base = atomicAdd(f.tier[t].count, (uint32_t)__popc(m));
-        base = __shfl_sync(kFull, base, __ffs(m) - 1);
-        if (tier == t) f.tier[t].ids[base + __popc(m & ((1u << lane) - 1u))] = x;
+      for (int q = 0; q < 4; ++q)
+        if (c0 + 8 * q < dg) push_entry(a, f, b + c0 + 8 * q);
+    }
+    __syncwarp();
+    for (uint32_t big = __ballot_sync(kFull, d > kPushRow && (lane & 7) == 0); big; big &= big - 1u) {
+      const int32_t rb = __shfl_sync(kFull, b, __ffs(big) - 1), rd = __shfl_sync(kFull, d, __ffs(big) - 1);
+      for (int64_t c0 = lane; c0 < rd; c0 += 128) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (c0 + 32 * q < rd) push_entry(a, f, (int32_t)(rb + c0 + 32 * q));
       }
     }
   }
 }
 
-// Changed vertices that are not recomputed keep their (new) label.
-__global__ void __launch_bounds__(256) k_frontier_copy(StepArgs a, Frontier f) {
+// Lists the marked vertices among [0, nscan) by tier, near id order (so that
+// the tiers walk their rows as they lie in memory), kListRound vertices a block
+// and round with one add per tier; then copies the changed vertices that are not
+// recomputed (they keep their new label) and sets the hubs' states: marked
+// hubs go through the majority check (2), the others are done (1).
+constexpr int kListItems = 8, kListRound = 256 * kListItems;
+__global__ void __launch_bounds__(256) k_frontier_list(StepArgs a, Frontier f, int32_t nscan, HubPlan hp) {
   if (step_mode(a) != kModeFrontier) return;
+  __shared__ uint32_t cnt[5], base[5];
+  const int lane = threadIdx.x & 31;
+  for (int64_t v0 = (int64_t)blockIdx.x * kListRound; v0 < nscan; v0 += (int64_t)gridDim.x * kListRound) {  // block-uniform
+    if (threadIdx.x < 5) cnt[threadIdx.x] = 0u;
+    __syncthreads();
+    int tier[kListItems];
+    uint32_t at[kListItems];
+#pragma unroll
+    for (int q = 0; q < kListItems; ++q) {
+      const int64_t v = v0 + q * 256 + threadIdx.x;
+      tier[q] = v < nscan && f.act[v] == f.epoch ? 0 : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < kListItems; ++q) {
+      const int64_t v = v0 + q * 256 + threadIdx.x;
+      if (tier[q] == 0) {
+        const int32_t d = a.off[v + 1] - a.off[v];
+        tier[q] = d <= f.tiny_max ? 0 : d <= 16 ? 1 : d <= 32 ? 2 : d <= f.mid_max ? 3 : d <= f.big_max ? 4 : -1;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kListItems; ++q) {
+      at[q] = 0;
+      for (uint32_t left = __ballot_sync(kFull, tier[q] >= 0); left;) {  // usually one tier a warp
+        const int t = __shfl_sync(kFull, tier[q], __ffs(left) - 1);
+        const uint32_t m = __ballot_sync(kFull, tier[q] == t);
+        uint32_t w = 0;
+        if (lane == __ffs(m) - 1) w = atomicAdd(&cnt[t], (uint32_t)__popc(m));
+        w = __shfl_sync(kFull, w, __ffs(m) - 1);
+        if (tier[q] == t) at[q] = w + __popc(m & ((1u << lane) - 1u));
+        left &= ~m;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < 5) base[threadIdx.x] = cnt[threadIdx.x] ? atomicAdd(f.tier[threadIdx.x].count, cnt[threadIdx.x]) : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kListItems; ++q)
+      if (tier[q] >= 0) f.tier[tier[q]].ids[base[tier[q]] + at[q]] = (int32_t)(v0 + q * 256 + threadIdx.x);
+    __syncthreads();  // base is read no more
+  }
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
   const uint32_t nc = *f.chg_in_n;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = t0; i < nc; i += nt) {
     const int32_t v = f.chg_in[i];
     if (f.act[v] != f.epoch) a.lout[v] = a.lin[v];
   }
-}
-
-// Marked hubs go through the majority check (state 2), unmarked ones are
-// done (state 1).
-__global__ void k_frontier_hubs(StepArgs a, Frontier f, HubPlan hp) {
-  if (step_mode(a) != kModeFrontier) return;
-  const int32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h < hp.nhubs) hp.hub_state[h] = f.act[hp.hub_v[h]] == f.epoch ? 2u : 1u;
+  for (int64_t h = t0; h < hp.nhubs; h += nt) hp.hub_state[h] = f.act[hp.hub_v[h]] == f.epoch ? 2u : 1u;
 }
 
 // Symmetry check of a CSR with strictly ascending rows, one thread per edge:
