@@ -46,7 +46,7 @@
 #include <vector>
 
 #include "../../include/glp.h"
-#include "device.cuh"
+#include "small_rows.cuh"
 #include "smem_attr.h"
 
 namespace glp {
@@ -80,7 +80,7 @@ struct BatchArgs {
   int64_t class_v[9];      // class c owns vertices [class_v[c], class_v[c+1])
   int64_t bstart[8][9];    // class c, bucket q: order[bstart[c][q], bstart[c][q+1])
   uint32_t mode;           // kB* strategy bits
-  uint32_t warp_words;     // shared words per warp for group tables
+  uint32_t warp_words;     // shared words per warp for staged rows or group tables
   uint32_t blk_cap;        // table slots of the block tier
   int32_t* lab0;
   int32_t* lab1;
@@ -152,18 +152,35 @@ __device__ __forceinline__ int32_t graph_of(const int64_t* base, int32_t ng, int
   return lo;
 }
 
+// Classic counts (small_rows.cuh, offer).
+struct CountScore {
+  static constexpr bool kKeep = false, kPacked = true, kScan = false, kLV = false;
+  __device__ __forceinline__ uint32_t key32(uint32_t k, int32_t) const { return k; }
+  __device__ __forceinline__ int64_t from_vol(uint32_t k, int32_t) const { return (int64_t)k; }
+  __device__ __forceinline__ int32_t vol_of(int32_t) const { return 0; }
+};
+
+// Table slots of a group: four a neighbour (a quarter-full table probes less),
+// two at the largest degrees, where a warp's slice holds no more.
+template <int G, int L>
+constexpr uint32_t group_slots() {
+  uint32_t p = 1;
+  while (p < 2u * G * L) p <<= 1;
+  return p < 512u ? 2 * p : p;
+}
+
 // One vertex per group of G lanes (G | 32), at most G*L neighbours, L labels
 // per lane in registers.  v < 0: this group has no vertex (it still takes
-// part in the warp-wide shuffles).  keys/vals: the group's table slice of
-// at least pow2(2*G*L) slots.  A strict majority of the own label decides
+// part in the warp-wide shuffles).  keys: the group's table slice, kCap =
+// group_slots<G, L>() slots of a key and a 16-bit count.  A strict majority of the own label decides
 // the vertex when `majority` is set; otherwise (or when it fails) the labels
 // are counted in the table, lanes holding the group leader's label adding
 // once through the leader.  Returns "changed" on the group leader.
 template <int G, int L>
 __device__ __forceinline__ bool group_vertex(const BatchArgs& a, int32_t v, const int32_t* __restrict__ lin,
-                                             int32_t* __restrict__ lout, uint32_t* keys, uint32_t* vals,
-                                             bool majority, const uint8_t* __restrict__ fin,
+                                             int32_t* __restrict__ lout, uint32_t* keys, bool majority, const uint8_t* __restrict__ fin,
                                              uint8_t* __restrict__ fout) {
+  constexpr uint32_t kCap = group_slots<G, L>();
   const int lane = threadIdx.x & 31;
   const int gl = lane & (G - 1);
   const uint32_t gmask = G == 32 ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
@@ -212,14 +229,14 @@ __device__ __forceinline__ bool group_vertex(const BatchArgs& a, int32_t v, cons
       done = true;
     }
   }
-  const uint32_t cap = done ? 0u : pow2_ceil(2u * (uint32_t)d);
+  // claim-first 16-bit counts; four slots a neighbour where they fit
+  const uint32_t cap = done ? 0u : min(pow2_ceil(4u * (uint32_t)d), kCap);
+  uint32_t* vals = keys + kCap;
   __syncwarp();
-  for (uint32_t s = gl; s < cap; s += G) {
-    keys[s] = 0;
-    vals[s] = 0;
-  }
+  for (uint32_t s = gl; s < cap; s += G) keys[s] = 0;
+  for (uint32_t s = gl; s < cap / 2; s += G) vals[s] = 0;
   __syncwarp();
-  Best best = best_none();
+  PackedCand best;
   bool fail = false;
 #pragma unroll
   for (int q = 0; q < L; ++q) {
@@ -233,30 +250,20 @@ __device__ __forceinline__ bool group_vertex(const BatchArgs& a, int32_t v, cons
       else if (has && lab[q] == l0) has = false;
     }
     if (has) {
-      const uint32_t tot = table_insert_bounded(keys, vals, cap - 1, (uint32_t)lab[q] + 1u, k, cap, nullptr, nullptr);
-      if (tot == kNoSlot) {
-        fail = true;
-      } else {
-        const Best c{(int64_t)tot, lab[q]};
-        if (better(c, best)) best = c;
-      }
+      const uint32_t tot = table_claim_insert<true>(keys, vals, cap - 1, (uint32_t)lab[q] + 1u, k, cap);
+      if (tot == kNoSlot) fail = true;
+      else offer(best, CountScore{}, tot, 0, lab[q]);
     }
   }
   if (fail) atomicOr(a.err, kErrProbe);
-  best = group_max<G>(best);
+  const uint32_t top = __reduce_max_sync(gmask, best.s);
+  const int32_t l = (int32_t)__reduce_max_sync(gmask, best.s == top ? best.l : 0u);
   if (done) return false;
   if (gl == 0) {
-    lout[v] = best.l;
-    fout[v] = best.l != own;
+    lout[v] = l;
+    fout[v] = l != own;
   }
-  return gl == 0 && best.l != own;
-}
-
-template <int G, int L>
-constexpr uint32_t group_slots() {  // pow2(2*G*L)
-  uint32_t p = 1;
-  while (p < 2u * G * L) p <<= 1;
-  return p;
+  return gl == 0 && l != own;
 }
 
 // Sweep order[lo, hi) with groups of G lanes; smem_warp: this warp's slice.
@@ -269,14 +276,13 @@ __device__ __forceinline__ uint32_t sweep_groups(const BatchArgs& a, int64_t lo,
   constexpr uint32_t kSlots = group_slots<G, L>();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = lane / G;
-  uint32_t* keys = smem_warp + (size_t)grp * 2 * kSlots;
-  uint32_t* vals = keys + kSlots;
+  uint32_t* keys = smem_warp + (size_t)grp * (kSlots + kSlots / 2);
   const int64_t nw = (int64_t)gridDim.x * (NT / 32);
   uint32_t chg = 0;
   for (int64_t i0 = lo + ((int64_t)blockIdx.x * (NT / 32) + warp) * kGroups; i0 < hi; i0 += nw * kGroups) {
     const int64_t i = i0 + grp;
     const int32_t v = i < hi ? a.order[i] : -1;
-    chg += group_vertex<G, L>(a, v, lin, lout, keys, vals, majority, fin, fout) ? 1u : 0u;
+    chg += group_vertex<G, L>(a, v, lin, lout, keys, majority, fin, fout) ? 1u : 0u;
   }
   return chg;
 }
@@ -351,55 +357,84 @@ __device__ __forceinline__ bool block_vertex(const BatchArgs& a, int32_t v, cons
   return threadIdx.x == 0 && best.l != lin[v];
 }
 
-// One vertex per thread (1 <= degree <= TT): its labels sorted in registers,
-// counts read off the runs (sort_keys).
-template <int TT>
-__device__ __forceinline__ bool thread_vertex(const BatchArgs& a, int32_t v, const int32_t* __restrict__ lin,
-                                              int32_t* __restrict__ lout, const uint8_t* __restrict__ fin,
-                                              uint8_t* __restrict__ fout) {
-  const int64_t b = a.off[v];
-  const int32_t d = (int32_t)(a.off[v + 1] - b);
-  int32_t lab[TT];
-#pragma unroll
-  for (int i = 0; i < TT; ++i) lab[i] = i < d ? ld_stream(a.cols + b + i) : -1;
-  if (fin) {  // no neighbour changed in the previous step: the label stays
-    bool any = false;
-#pragma unroll
-    for (int i = 0; i < TT; ++i)
-      if (lab[i] >= 0) any = any || fin[lab[i]] != 0;
-    if (!any) {
-      lout[v] = lin[v];
-      fout[v] = 0;
-      return false;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < TT; ++i) lab[i] = lab[i] >= 0 ? ld_label(lin + lab[i]) : INT32_MAX;
-  sort_keys(lab);
-  Best best = best_none();
-  uint32_t run = 0;
-#pragma unroll
-  for (int i = 0; i < TT; ++i) {
-    run = (i > 0 && lab[i] == lab[i > 0 ? i - 1 : 0]) ? run + 1u : 1u;
-    const bool end = (i == TT - 1) || lab[(i + 1) & (TT - 1)] != lab[i];
-    if (end && lab[i] != INT32_MAX) {
-      const Best c{(int64_t)run, lab[i]};
-      if (better(c, best)) best = c;
-    }
-  }
-  const int32_t own = lin[v];
-  lout[v] = best.l;
-  fout[v] = best.l != own;
-  return best.l != own;
-}
-
-template <int NT, int TT>
+// Sweep order[lo, hi), degrees 1..R, one vertex per thread: the warp loads its
+// 32 rows together (eight lanes a row; small_rows.cuh), then each thread sorts
+// its labels in registers and reads the counts off the runs.  A thread loading
+// its own row, 32 sectors a load, and sorting with a bitonic network took
+// MEASURED_BATCH.
+template <int NT, int R>
 __device__ __forceinline__ uint32_t sweep_threads(const BatchArgs& a, int64_t lo, int64_t hi,
                                                   const int32_t* __restrict__ lin, int32_t* __restrict__ lout,
-                                                  const uint8_t* fin, uint8_t* fout) {
+                                                  uint32_t* slab, const uint8_t* fin, uint8_t* fout) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane >> 3;
   uint32_t chg = 0;
-  for (int64_t i = lo + (int64_t)blockIdx.x * NT + threadIdx.x; i < hi; i += (int64_t)gridDim.x * NT)
-    chg += thread_vertex<TT>(a, a.order[i], lin, lout, fin, fout) ? 1u : 0u;
+  for (int64_t i0 = lo + (int64_t)blockIdx.x * NT + warp * 32; i0 < hi; i0 += (int64_t)gridDim.x * NT) {  // warp-uniform
+    int32_t v = -1, own = 0, d = 0;
+    int64_t b = 0;
+    if (i0 + lane < hi) {
+      v = a.order[i0 + lane];
+      own = lin[v];
+      b = a.off[v];
+      d = (int32_t)(a.off[v + 1] - b);
+    }
+    const int dmax = (int)__reduce_max_sync(kFull, (uint32_t)d);
+    __syncwarp();  // the slab is read no more
+    // all columns first, which takes no registers
+#pragma unroll 1
+    for (int c0 = 0; c0 < dmax; c0 += 8) {
+      const int i = c0 + (lane & 7);
+#pragma unroll
+      for (int g = 0; g < 8; ++g) {
+        const int64_t rb = __shfl_sync(kFull, b, 4 * g + grp);
+        if (i < __shfl_sync(kFull, d, 4 * g + grp)) async_word(slab + small_at<R>(4 * g + grp, i), a.cols + rb + i);
+      }
+    }
+    async_wait();
+    // rows with a changed neighbour, bit t: thread t's (every row without flags);
+    // a row without one keeps its label (exact: its neighbourhood is what it was)
+    uint32_t rows = kFull;
+    if (fin) {
+      rows = 0u;
+      for (int c0 = 0; c0 < dmax; c0 += 8) {
+        const int i = c0 + (lane & 7);
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const bool in = i < __shfl_sync(kFull, d, 4 * g + grp);
+          const uint32_t m = __ballot_sync(kFull, in && fin[slab[small_at<R>(4 * g + grp, i)]] != 0);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) rows |= (m >> (8 * q) & 0xffu) ? 1u << (4 * g + q) : 0u;
+        }
+      }
+    }
+    if (rows) {  // warp-uniform
+#pragma unroll 1
+      for (int c0 = 0; c0 < dmax; c0 += 8) {
+        const int i = c0 + (lane & 7);
+        int32_t lab[8];
+        bool in[8];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const int t = 4 * g + grp;
+          in[g] = i < __shfl_sync(kFull, d, t) && (rows >> t & 1u);
+          if (in[g]) lab[g] = ld_label(lin + slab[small_at<R>(t, i)]);
+        }
+#pragma unroll
+        for (int g = 0; g < 8; ++g)
+          if (in[g]) slab[small_at<R>(4 * g + grp, i)] = (uint32_t)lab[g];
+      }
+    }
+    __syncwarp();
+    int32_t best = own;
+    if (rows) {
+      const int32_t l = small_row_best<R, false, CountScore, int32_t>(CountScore{}, slab, lane, d, dmax);
+      if (rows >> lane & 1u) best = l;
+    }
+    if (v >= 0) {
+      lout[v] = best;
+      fout[v] = best != own;
+      chg += best != own ? 1u : 0u;
+    }
+  }
   return chg;
 }
 
@@ -484,11 +519,11 @@ __global__ void __launch_bounds__(NT) k_batch(BatchArgs a) {
       chg += sweep_groups<NT, 32, 4>(a, B[2], B[3], lin, lout, smem_warp, majority, fin, fout);
       if (a.mode & kB3Half) chg += sweep_groups<NT, 16, 4>(a, B[3], B[4], lin, lout, smem_warp, majority, fin, fout);
       else chg += sweep_groups<NT, 32, 2>(a, B[3], B[4], lin, lout, smem_warp, majority, fin, fout);
-      if (a.mode & kB4Threads) chg += sweep_threads<NT, 32>(a, B[4], B[5], lin, lout, fin, fout);
+      if (a.mode & kB4Threads) chg += sweep_threads<NT, 32>(a, B[4], B[5], lin, lout, smem_warp, fin, fout);
       else chg += sweep_groups<NT, 8, 4>(a, B[4], B[5], lin, lout, smem_warp, majority, fin, fout);
-      if (a.mode & kB5Threads) chg += sweep_threads<NT, 16>(a, B[5], B[6], lin, lout, fin, fout);
+      if (a.mode & kB5Threads) chg += sweep_threads<NT, 16>(a, B[5], B[6], lin, lout, smem_warp, fin, fout);
       else chg += sweep_groups<NT, 4, 4>(a, B[5], B[6], lin, lout, smem_warp, majority, fin, fout);
-      chg += sweep_threads<NT, 8>(a, B[6], B[7], lin, lout, fin, fout);
+      chg += sweep_threads<NT, 8>(a, B[6], B[7], lin, lout, smem_warp, fin, fout);
     }
     block_count_add<NT>(a.changed + it, chg, red_u);
     if (it + 1 < a.niter && !grid_barrier(a.bar, ++phase * gridDim.x, a.err, a.barrier_ns)) return;
@@ -763,7 +798,11 @@ BatchArgs make_args(glp_batch* b, const Config& c, int32_t niter) {
   }
   for (int k = 0; k <= b->nclass; ++k) a.class_v[k] = b->class_v[k];
   a.mode = (c.tt >= 32 ? kB4Threads : 0u) | (c.tt >= 16 ? kB5Threads : 0u) | (c.half ? kB3Half : 0u);
-  a.warp_words = max_degree_in(b, 128, 256) ? 2 * group_slots<32, 8>() : 2 * group_slots<32, 4>();
+  // a warp's 32 staged rows, or the tables of its groups (all alike)
+  static_assert(group_slots<32, 8>() == group_slots<32, 4>() && 2 * group_slots<16, 4>() == group_slots<32, 4>() &&
+                    4 * group_slots<8, 4>() == group_slots<32, 4>() && 8 * group_slots<4, 4>() == group_slots<32, 4>(),
+                "one slice serves every group size");
+  a.warp_words = std::max<uint32_t>(32u * (uint32_t)c.tt, group_slots<32, 4>() * 3 / 2);
   const int bdeg = max_degree_in(b, 256, kBatchMaxDegree);
   a.blk_cap = bdeg ? pow2_host(2u * (uint32_t)bdeg) : 0u;
   a.lab0 = b->d_lab[0];
