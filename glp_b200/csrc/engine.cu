@@ -193,10 +193,17 @@ void build_host_plan(const int32_t* off, int32_t n, const TierParams& t, HostPla
     } else if (d <= t.mid_max) {
       hp->mid.push_back(v);
       hp->mb.push_back(v);
+      if (d <= kPairDegree) {
+        hp->pair.push_back(v);
+      } else {
+        hp->mid_rest.push_back(v);
+        hp->mb_rest.push_back(v);
+      }
       tier = 4;
     } else if (d <= t.big_max) {
       hp->big.push_back(v);
       hp->mb.push_back(v);
+      hp->mb_rest.push_back(v);
       int r = 0;
       while (r + 1 < kBigParts && d > kBigPartMax[r]) ++r;
       hp->big_part[r].push_back(v);
@@ -296,7 +303,7 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     // over the non-increasing degrees; only the hubs' offsets reach the host
     // thresholds, descending: big_max, the part bounds below it, mid_max, 32,
     // 16, tiny_max, 0; b[i] = vertices of degree > thr[i]
-    constexpr int kT = kBigParts + 5;
+    constexpr int kT = kBigParts + 6;
     int32_t thr[kT];
     thr[0] = t.big_max;
     for (int r = kBigParts - 2, i = 1; r >= 0; --r, ++i) thr[i] = std::min<int32_t>(kBigPartMax[r], t.big_max);
@@ -305,6 +312,7 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     thr[kBigParts + 2] = 16;
     thr[kBigParts + 3] = t.tiny_max;
     thr[kBigParts + 4] = 0;
+    thr[kBigParts + 5] = std::min<int32_t>(kPairDegree, t.mid_max);
     int32_t b[kT];
     if ((rc = device_bounds(g, thr, kT, b))) return rc;
     for (int i = 1; i < kBigParts; ++i) b[i] = std::min(std::max(b[i], b[i - 1]), b[kBigParts]);
@@ -315,6 +323,9 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     p.big = range_verts(b[0], b[kBigParts]);
     p.mid = range_verts(b[kBigParts], b[kBigParts + 1]);
     p.mb = range_verts(b[0], b[kBigParts + 1]);
+    p.pair = range_verts(b[kBigParts + 5], b[kBigParts + 1]);
+    p.mid_rest = range_verts(b[kBigParts], b[kBigParts + 5]);
+    p.mb_rest = range_verts(b[0], b[kBigParts + 5]);
     p.g32 = range_verts(b[kBigParts + 1], b[kBigParts + 2]);
     p.g16 = range_verts(b[kBigParts + 2], b[kBigParts + 3]);
     p.tiny = range_verts(b[kBigParts + 3], b[kBigParts + 4]);
@@ -325,7 +336,9 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     p.isolated = hp.isolated;
     if ((rc = upload_verts(&p, hp.tiny, &p.tiny)) || (rc = upload_verts(&p, hp.g16, &p.g16)) ||
         (rc = upload_verts(&p, hp.g32, &p.g32)) || (rc = upload_verts(&p, hp.mid, &p.mid)) ||
-        (rc = upload_verts(&p, hp.big, &p.big)) || (rc = upload_verts(&p, hp.mb, &p.mb))) {
+        (rc = upload_verts(&p, hp.big, &p.big)) || (rc = upload_verts(&p, hp.mb, &p.mb)) ||
+        (rc = upload_verts(&p, hp.pair, &p.pair)) || (rc = upload_verts(&p, hp.mid_rest, &p.mid_rest)) ||
+        (rc = upload_verts(&p, hp.mb_rest, &p.mb_rest))) {
       free_plan(&p);
       return rc;
     }
@@ -538,10 +551,14 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     *launches += 6;
     if ((rc = mark_on(L.aux[0], 5, 1))) return rc;
   }
-  if (L.allow_majority && modal && p.mb.n) {
+  // unweighted classic-type scores count the mid tier's rows up to kPairDegree
+  // by k_pair in full and majority steps
+  constexpr bool kPair = !W && S::kPacked && !S::kScan;
+  const Verts& mb = kPair ? p.mb_rest : p.mb;
+  if (L.allow_majority && modal && mb.n) {
     if ((rc = mark_on(s, 7, 0))) return rc;  // slot 7: the majority pre-pass
-    k_major_warp<W><<<(unsigned)std::min<int64_t>(cdiv((int64_t)p.mb.n * 32, 256), kMaxGrid), 256, 0, s>>>(
-        a, p.mb, p.tiers.mid_max, p.fmid, p.fbig);
+    k_major_warp<W><<<(unsigned)std::min<int64_t>(cdiv((int64_t)mb.n * 32, 256), kMaxGrid), 256, 0, s>>>(
+        a, mb, p.tiers.mid_max, p.fmid, p.fbig);
     if ((rc = mark_on(s, 7, 1))) return rc;
     ++*launches;
   }
@@ -635,9 +652,22 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
   }
   if (p.mid.n) {
     if ((rc = mark_on(s, 3, 0))) return rc;
+    // (frontier lists hold the pair rows too: the grid is for the whole tier)
     const unsigned grid = (unsigned)std::min<int64_t>(cdiv(p.mid.n, kMidNT / 32), kMaxGrid);
     bool c16w = false;  // weighted classic with small weight sums: 16-bit counts
-    const TierWork mw = work(p.mid, 3, &p.fmid);
+    const TierWork mw = work(kPair ? p.mid_rest : p.mid, 3, &p.fmid);
+    if constexpr (kPair) {
+      if (p.pair.n) {
+        // beside the big tier where there is one, else beside the small tiers
+        // (SLPA 2M 3.95 ms a run against 4.24 the other way); within the mid
+        // tier's events when timed
+        cudaStream_t ps = L.ev || !p.big.n ? s : L.aux[1];
+        const size_t sm = (size_t)(kSmallNT / 32) * small_words<32, false, S>() * sizeof(uint32_t);
+        k_pair<S><<<(unsigned)std::min<int64_t>(cdiv((int64_t)p.pair.n * 2, kSmallNT), kMaxGrid), kSmallNT, sm, ps>>>(
+            a, TierWork{p.pair, FailList{nullptr, nullptr}, FailList{nullptr, nullptr}, 2}, score);
+        ++*launches;
+      }
+    }
     if constexpr (W && S::kPacked) {
       c16w = p.mid_c16;
       if (c16w) k_mid<kMidCap, kMidNT, W, S, true><<<grid, kMidNT, 0, s>>>(a, mw, score);

@@ -57,6 +57,7 @@ int tiers_for_graph(const glp_params* p, bool weighted, TierParams* t);
 // Host-side plan (pure function of the offsets and the tier parameters).
 struct HostPlan {
   std::vector<int32_t> tiny, g16, g32, mid, big, mb;  // vertex lists (ascending ids); mb = mid + big
+  std::vector<int32_t> pair, mid_rest, mb_rest;        // mid up to kPairDegree, mid and mb above it
   std::vector<int32_t> big_part[kBigParts];            // the big tier by kBigPartMax range
   int64_t isolated = 0;
   int64_t edges[7] = {0, 0, 0, 0, 0, 0, 0};  // per tier, as the vertex counts of glp_graph_plan
@@ -74,7 +75,7 @@ struct DevicePlan {
   cudaStream_t setup = nullptr;  // stream of the set-up copies (the handle's)
   TierParams tiers;
   bool valid = false;
-  Verts tiny{}, g16{}, g32{}, mid{}, big{}, mb{}, big_part[kBigParts]{};
+  Verts tiny{}, g16{}, g32{}, mid{}, big{}, mb{}, pair{}, mid_rest{}, mb_rest{}, big_part[kBigParts]{};
   FailList fmid{}, fbig{};
   FailList fscreen{};  // big-tier vertices a summary screen left to the exact kernel
   // list counters: [majority mid, majority big, frontier tiny, g16, g32, mid,

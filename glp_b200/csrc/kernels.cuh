@@ -192,17 +192,18 @@ struct TierWork {
   Verts all;
   FailList major;  // ids == nullptr: the tier has no pre-pass
   FailList front;
-  int full_only;   // 1: works only in full mode (a sub-range of a tier)
+  int full_only;   // a sub-range of a tier: 1 works only in full mode, 2 in full and majority mode
   int listed = 0;  // 1: works on the `major` list in every mode (screen fallbacks)
   __device__ __forceinline__ int32_t size(int32_t mode) const {
     if (listed) return (int32_t)*major.count;
-    if (full_only) return mode == kModeFull ? all.n : 0;
+    if (full_only) return mode == kModeFull || (full_only == 2 && mode == kModeMajority) ? all.n : 0;
     if (mode == kModeFrontier && front.ids) return (int32_t)*front.count;
     if (mode == kModeMajority && major.ids) return (int32_t)*major.count;
     return all.n;
   }
   __device__ __forceinline__ int32_t at(int32_t mode, int64_t i) const {
     if (listed) return major.ids[i];
+    if (full_only) return all[i];
     if (mode == kModeFrontier && front.ids) return front.ids[i];
     if (mode == kModeMajority && major.ids) return major.ids[i];
     return all[i];
@@ -378,13 +379,81 @@ constexpr int small_blocks() {
   constexpr int n = 221184 / (kSmallNT / 32 * small_words<R, W, S>() * 4 + 1024);
   return n < 4 ? n : 4;
 }
+// Stages the warp's 32 rows (lane t's: d entries from b, d <= R; dmax = the
+// largest d): labels, and weights and volumes where the score has them.
+template <int R, bool W, class S>
+__device__ __forceinline__ void stage_rows(const StepArgs& a, const S& score, uint32_t* slab, int32_t b, int32_t d,
+                                           int dmax) {
+  const int lane = threadIdx.x & 31;
+  uint32_t* sw = slab + 32 * R;
+  uint32_t* svol = slab + 32 * R * (W ? 2 : 1);
+      // a lane helps to load rows 4g + lane / 8, eight of them in flight
+      const int grp = lane >> 3;
+      if constexpr (R < 32 || W || S::kLV) {
+        // all columns (and weights) first, which takes no registers, then the
+        // labels; a lane gathers for what it copied.  (Fewer rounds of latency:
+        // weighted layered planted 2M 19.1 -> 17.2 ms; degrees 17..32 with labels
+        // alone have warps enough to hide them and ran 3 % slower so.)
+#pragma unroll 1
+        for (int c0 = 0; c0 < dmax; c0 += 8) {
+          const int i = c0 + (lane & 7);
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            const int32_t rb = __shfl_sync(kFull, b, 4 * g + grp), rd = __shfl_sync(kFull, d, 4 * g + grp);
+            if (i < rd) {
+              const int at = small_at<R>(4 * g + grp, i);
+              async_word(slab + at, a.cols + rb + i);
+              if (W) async_word(sw + at, a.w + rb + i);
+            }
+          }
+        }
+        async_wait();
+#pragma unroll 1
+        for (int c0 = 0; c0 < dmax; c0 += 8) {
+          const int i = c0 + (lane & 7);
+          int32_t lab[8], vl[8];
+          bool in[8];
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            in[g] = i < __shfl_sync(kFull, d, 4 * g + grp);
+            if (in[g]) score.load(a, (int32_t)slab[small_at<R>(4 * g + grp, i)], lab[g], vl[g]);
+          }
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            if (in[g]) {
+              const int at = small_at<R>(4 * g + grp, i);
+              slab[at] = (uint32_t)lab[g];
+              if (S::kLV) svol[at] = (uint32_t)vl[g];
+            }
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (int c0 = 0; c0 < dmax; c0 += 8) {
+          const int i = c0 + (lane & 7);
+          int32_t lab[8], vl[8];
+          bool in[8];
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            const int32_t j = __shfl_sync(kFull, b, 4 * g + grp) + i;
+            in[g] = i < __shfl_sync(kFull, d, 4 * g + grp);
+            lab[g] = in[g] ? ld_stream(a.cols + j) : -1;
+          }
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            if (in[g]) score.load(a, lab[g], lab[g], vl[g]);
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            if (in[g]) slab[small_at<R>(4 * g + grp, i)] = (uint32_t)lab[g];
+        }
+      }
+}
+
 template <int R, bool W, class S, class K>
 __global__ void __launch_bounds__(kSmallNT, sizeof(K) == 4 ? small_blocks<R, W, S>() : 2) k_small(StepArgs a, TierWork tw, S score) {
   extern __shared__ __align__(16) uint32_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t* slab = smem + warp * small_words<R, W, S>();
-  uint32_t* sw = slab + 32 * R;
-  uint32_t* svol = slab + 32 * R * (W ? 2 : 1);
   const int32_t mode = step_mode(a);
   const int32_t nwork = tw.size(mode);
   const int64_t stride = (int64_t)gridDim.x * kSmallNT;
@@ -402,71 +471,54 @@ __global__ void __launch_bounds__(kSmallNT, sizeof(K) == 4 ? small_blocks<R, W, 
       d = fixed ? 0 : a.off[v + 1] - b;
     }
     const int dmax = (int)__reduce_max_sync(kFull, (uint32_t)d);
-    // a lane helps to load rows 4g + lane / 8, eight of them in flight
-    const int grp = lane >> 3;
-    if constexpr (R < 32 || W || S::kLV) {
-      // all columns (and weights) first, which takes no registers, then the
-      // labels; a lane gathers for what it copied.  (Fewer rounds of latency:
-      // weighted layered planted 2M 19.1 -> 17.2 ms; degrees 17..32 with labels
-      // alone have warps enough to hide them and ran 3 % slower so.)
-#pragma unroll 1
-      for (int c0 = 0; c0 < dmax; c0 += 8) {
-        const int i = c0 + (lane & 7);
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const int32_t rb = __shfl_sync(kFull, b, 4 * g + grp), rd = __shfl_sync(kFull, d, 4 * g + grp);
-          if (i < rd) {
-            const int at = small_at<R>(4 * g + grp, i);
-            async_word(slab + at, a.cols + rb + i);
-            if (W) async_word(sw + at, a.w + rb + i);
-          }
-        }
-      }
-      async_wait();
-#pragma unroll 1
-      for (int c0 = 0; c0 < dmax; c0 += 8) {
-        const int i = c0 + (lane & 7);
-        int32_t lab[8], vl[8];
-        bool in[8];
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          in[g] = i < __shfl_sync(kFull, d, 4 * g + grp);
-          if (in[g]) score.load(a, (int32_t)slab[small_at<R>(4 * g + grp, i)], lab[g], vl[g]);
-        }
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          if (in[g]) {
-            const int at = small_at<R>(4 * g + grp, i);
-            slab[at] = (uint32_t)lab[g];
-            if (S::kLV) svol[at] = (uint32_t)vl[g];
-          }
-        }
-      }
-    } else {
-#pragma unroll 1
-      for (int c0 = 0; c0 < dmax; c0 += 8) {
-        const int i = c0 + (lane & 7);
-        int32_t lab[8], vl[8];
-        bool in[8];
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const int32_t j = __shfl_sync(kFull, b, 4 * g + grp) + i;
-          in[g] = i < __shfl_sync(kFull, d, 4 * g + grp);
-          lab[g] = in[g] ? ld_stream(a.cols + j) : -1;
-        }
-#pragma unroll
-        for (int g = 0; g < 8; ++g)
-          if (in[g]) score.load(a, lab[g], lab[g], vl[g]);
-#pragma unroll
-        for (int g = 0; g < 8; ++g)
-          if (in[g]) slab[small_at<R>(4 * g + grp, i)] = (uint32_t)lab[g];
-      }
-    }
+    stage_rows<R, W>(a, score, slab, b, d, dmax);
     __syncwarp();
     int32_t best = small_row_best<R, W, S, K>(score, slab, lane, d, dmax);
     if (best < 0) best = cur;  // a seed, or no labelled neighbour
     if (has) a.lout[v] = best;
     note_changes(a, notes, has && best != cur, v);
+    __syncwarp();  // the words are stored for the next vertices
+  }
+  tally_changes(a, notes);
+}
+
+// Degrees 33..kPairDegree of unweighted classic-type scores, outside frontier
+// steps: two lanes per vertex, half the row each (so a half is a row of
+// k_small).  Sorting takes about two warp instructions an entry where k_mid's
+// table takes four to six, and no atomics: SLPA on the overlapping 2M graph
+// (degrees 33..50) 81 -> 47 us a step, less than the majority pre-pass and
+// k_mid took together (144 us), so majority steps count these rows too.  More
+// lanes a row (65..1024, tried) gain nothing over the tables: the merge's
+// shuffles, one a clock per SM, grow with each doubling, and so they do with
+// weights or volumes to look up.
+constexpr int kPairDegree = 64;
+template <class S>
+__global__ void __launch_bounds__(kSmallNT, 4) k_pair(StepArgs a, TierWork tw, S score) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & 1;
+  uint32_t* slab = smem + warp * small_words<32, false, S>();
+  const int32_t mode = step_mode(a);
+  const int32_t nwork = tw.size(mode);
+  const int64_t stride = (int64_t)gridDim.x * (kSmallNT / 2);
+  ChangeNotes notes(a);
+  for (int64_t i0 = (int64_t)blockIdx.x * (kSmallNT / 2) + warp * 16; i0 < nwork; i0 += stride) {  // warp-uniform
+    const int64_t i = i0 + lane / 2;
+    const bool has = i < nwork;
+    int32_t v = 0, b = 0, dv = 0, cur = 0;
+    if (has) {
+      v = tw.at(mode, i);
+      cur = a.lcur[v];
+      b = a.off[v];
+      if (!(S::kKeep && score.fixed(v))) dv = a.off[v + 1] - b;
+    }
+    const int half = (dv + 1) / 2, d = sub ? dv - half : half;
+    const int dmax = (int)__reduce_max_sync(kFull, (uint32_t)d);
+    stage_rows<32, false>(a, score, slab, b + sub * half, d, dmax);
+    __syncwarp();
+    const unsigned long long best = pair_best(score, slab, lane, d, dmax);
+    const int32_t l = S::kKeep && !best ? cur : (int32_t)(uint32_t)best;
+    if (has && !sub) a.lout[v] = l;
+    note_changes(a, notes, has && !sub && l != cur, v);
     __syncwarp();  // the words are stored for the next vertices
   }
   tally_changes(a, notes);

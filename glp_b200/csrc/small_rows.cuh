@@ -1,6 +1,6 @@
-// small_rows.cuh -- rows of up to 32 entries, one per thread, staged in shared
-// memory by the warp (kernels.cuh, k_small; batch.cu): where an entry sits, and
-// the row's best label by sorting.
+// small_rows.cuh -- rows staged in shared memory by the warp, up to 32 entries
+// a lane (kernels.cuh, k_small and k_pair; batch.cu): where an entry sits, and
+// the row's best label by sorting, for a row per lane and a row per two lanes.
 #pragma once
 #include <type_traits>
 
@@ -109,6 +109,79 @@ __device__ __forceinline__ int32_t small_row_best(const S& score, const uint32_t
            : dmax <= 28 ? small_best<28, R, W, S, K>(score, slab, t, d)
                         : small_best<32, R, W, S, K>(score, slab, t, d);
   }
+}
+
+// Sorts the first N of 32 keys; the others are the largest key already.
+template <int N>
+__device__ __forceinline__ void sort_first(int32_t (&x)[32]) {
+  int32_t y[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) y[i] = x[i];
+  sort_keys(y);
+#pragma unroll
+  for (int i = 0; i < N; ++i) x[i] = y[i];
+}
+
+// The best (key, label) of a row over two lanes (lane, lane ^ 1), as key << 32 |
+// label on both; labels alone (no weights or volumes), 0 when none is labelled
+// (scores with kKeep).  The lane holds d <= 32 of the entries, dmax = the
+// warp's largest d.  Each lane sorts its own, one exchange in opposite order
+// leaves the smaller half of all keys on the even lane, five bitonic rounds
+// sort each half, and each lane reads the counts off its runs; the odd lane's
+// first run goes on from the even lane's last.
+template <class S>
+__device__ __forceinline__ unsigned long long pair_best(const S& score, const uint32_t* slab, int lane, int d,
+                                                        int dmax) {
+  static_assert(S::kPacked && !S::kScan, "counts alone");
+  int32_t key[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    key[i] = INT32_MAX;
+    if (i < d) {
+      const int32_t l = (int32_t)slab[small_at<32>(lane, i)];
+      if (!S::kKeep || l >= 0) key[i] = l;  // unlabelled: no entry
+    }
+  }
+  if (dmax <= 20) sort_first<20>(key);
+  else if (dmax <= 24) sort_first<24>(key);
+  else if (dmax <= 28) sort_first<28>(key);
+  else sort_first<32>(key);
+  const bool low = (lane & 1) == 0;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int32_t p = __shfl_xor_sync(kFull, key[31 - i], 1), q = __shfl_xor_sync(kFull, key[i], 1);
+    key[i] = low ? min(key[i], p) : max(key[i], p);
+    key[31 - i] = low ? min(key[31 - i], q) : max(key[31 - i], q);
+  }
+#pragma unroll
+  for (int j = 16; j >= 1; j /= 2)
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if ((i & j) == 0) {
+        const int32_t lo = min(key[i], key[i + j]), hi = max(key[i], key[i + j]);
+        key[i] = lo;
+        key[i + j] = hi;
+      }
+  // the even lane's last run, where the odd lane's first label continues it
+  uint32_t tail = 1;
+#pragma unroll
+  for (int i = 1; i < 32; ++i) tail = key[i] == key[i - 1] ? tail + 1u : 1u;
+  const int32_t before = __shfl_up_sync(kFull, key[31], 1);
+  const uint32_t carry = __shfl_up_sync(kFull, tail, 1);
+  uint32_t run = !low && key[0] == before ? carry : 0u;
+  PackedCand best;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    if (i > 0 && key[i] != key[i > 0 ? i - 1 : 0]) run = 0;
+    ++run;
+    const uint32_t c = score.key32(run, 0);
+    if (key[i] != INT32_MAX && c >= best.s) {  // labels ascend: equal keys take the later
+      best.s = c;
+      best.l = (uint32_t)key[i];
+    }
+  }
+  const unsigned long long mine = ((unsigned long long)best.s << 32) | best.l;
+  return max(mine, __shfl_xor_sync(kFull, mine, 1));
 }
 
 }  // namespace glp
