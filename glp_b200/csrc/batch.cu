@@ -18,13 +18,15 @@
 // grid-stride sweeps over that order:
 //   block tier  (WMAX < d <= 4096): a CTA per vertex, shared table of
 //                                   pow2(2d) slots;
-//   warp tier   (TT < d <= WMAX)  : a warp per vertex, its <= 8 labels per
+//   warp tier   (64 < d <= WMAX)  : a warp per vertex, its <= 8 labels per
 //                                   lane held in registers: a strict-majority
 //                                   test of the own label, else a per-warp
 //                                   shared table;
-//   thread tier (1 <= d <= TT)    : a thread per vertex, labels sorted in
-//                                   registers (sorting network), counts read
-//                                   off the runs.
+//   thread tier (1 <= d <= 64)    : a thread per vertex (two above degree 32),
+//                                   labels sorted in registers (sorting
+//                                   network), counts read off the runs.
+// (A run's parameters may count degrees 9..32 by lane groups and 33..64 by
+// warps, with tables.)
 // Every step also writes a change flag per vertex (1 byte).  Once few labels
 // still change (fewer than frontier_permille, default 10, per 1000 vertices
 // in the previous step), a vertex first reads
@@ -156,8 +158,6 @@ __device__ __forceinline__ int32_t graph_of(const int64_t* base, int32_t ng, int
 struct CountScore {
   static constexpr bool kKeep = false, kPacked = true, kScan = false, kLV = false;
   __device__ __forceinline__ uint32_t key32(uint32_t k, int32_t) const { return k; }
-  __device__ __forceinline__ int64_t from_vol(uint32_t k, int32_t) const { return (int64_t)k; }
-  __device__ __forceinline__ int32_t vol_of(int32_t) const { return 0; }
 };
 
 // Table slots of a group: four a neighbour (a quarter-full table probes less),
@@ -357,25 +357,33 @@ __device__ __forceinline__ bool block_vertex(const BatchArgs& a, int32_t v, cons
   return threadIdx.x == 0 && best.l != lin[v];
 }
 
-// Sweep order[lo, hi), degrees 1..R, one vertex per thread: the warp loads its
-// 32 rows together (eight lanes a row; small_rows.cuh), then each thread sorts
+// Sweep order[lo, hi), degrees 1..R, one vertex per thread (L = 2: degrees up to
+// 2R, a vertex per two threads, half the row each): the warp loads its 32 rows
+// together (eight lanes a row; small_rows.cuh), then each thread sorts
 // its labels in registers and reads the counts off the runs.  A thread loading
-// its own row, 32 sectors a load, and sorting with a bitonic network took
-// MEASURED_BATCH.
-template <int NT, int R>
+// its own row, 32 sectors a load, and sorting with a bitonic network, and
+// 16-lane groups with a count table for degrees 33..64, took 38.7 ms for 256
+// planted graphs and 20 steps (4.8 G entries); these sweeps take 24.1.
+template <int NT, int R, int L = 1>
 __device__ __forceinline__ uint32_t sweep_threads(const BatchArgs& a, int64_t lo, int64_t hi,
                                                   const int32_t* __restrict__ lin, int32_t* __restrict__ lout,
                                                   uint32_t* slab, const uint8_t* fin, uint8_t* fout) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane >> 3;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane >> 3, sub = lane & (L - 1);
   uint32_t chg = 0;
-  for (int64_t i0 = lo + (int64_t)blockIdx.x * NT + warp * 32; i0 < hi; i0 += (int64_t)gridDim.x * NT) {  // warp-uniform
+  for (int64_t i0 = lo + ((int64_t)blockIdx.x * NT + warp * 32) / L; i0 < hi;
+       i0 += (int64_t)gridDim.x * NT / L) {  // warp-uniform
     int32_t v = -1, own = 0, d = 0;
     int64_t b = 0;
-    if (i0 + lane < hi) {
-      v = a.order[i0 + lane];
+    if (i0 + lane / L < hi) {
+      v = a.order[i0 + lane / L];
       own = lin[v];
       b = a.off[v];
       d = (int32_t)(a.off[v + 1] - b);
+      if (L == 2) {
+        const int32_t half = (d + 1) / 2;
+        b += sub * half;
+        d = sub ? d - half : half;
+      }
     }
     const int dmax = (int)__reduce_max_sync(kFull, (uint32_t)d);
     __syncwarp();  // the slab is read no more
@@ -405,6 +413,7 @@ __device__ __forceinline__ uint32_t sweep_threads(const BatchArgs& a, int64_t lo
           for (int q = 0; q < 4; ++q) rows |= (m >> (8 * q) & 0xffu) ? 1u << (4 * g + q) : 0u;
         }
       }
+      if (L == 2) rows |= (rows & 0x55555555u) << 1 | (rows >> 1 & 0x55555555u);  // either half
     }
     if (rows) {  // warp-uniform
 #pragma unroll 1
@@ -426,10 +435,12 @@ __device__ __forceinline__ uint32_t sweep_threads(const BatchArgs& a, int64_t lo
     __syncwarp();
     int32_t best = own;
     if (rows) {
-      const int32_t l = small_row_best<R, false, CountScore, int32_t>(CountScore{}, slab, lane, d, dmax);
+      int32_t l;
+      if constexpr (L == 2) l = (int32_t)(uint32_t)pair_best(CountScore{}, slab, lane, d, dmax);
+      else l = small_row_best<R, false, CountScore, int32_t>(CountScore{}, slab, lane, d, dmax);
       if (rows >> lane & 1u) best = l;
     }
-    if (v >= 0) {
+    if (v >= 0 && sub == 0) {
       lout[v] = best;
       fout[v] = best != own;
       chg += best != own ? 1u : 0u;
@@ -456,7 +467,7 @@ __device__ __forceinline__ void block_count_add(unsigned long long* counter, uin
 // Strategy bits of a run (how buckets 3..5 are counted).
 constexpr uint32_t kB4Threads = 1u;  // degrees 17..32: a thread each (else 8-lane groups)
 constexpr uint32_t kB5Threads = 2u;  // degrees 9..16: a thread each (else 4-lane groups)
-constexpr uint32_t kB3Half = 4u;     // degrees 33..64: 16-lane groups (else whole warps)
+constexpr uint32_t kB3Half = 4u;     // degrees 33..64: two threads each (else whole warps)
 
 template <int NT>
 __global__ void __launch_bounds__(NT) k_batch(BatchArgs a) {
@@ -517,7 +528,7 @@ __global__ void __launch_bounds__(NT) k_batch(BatchArgs a) {
         chg += block_vertex<NT>(a, a.order[i], lin, lout, smem, red, fin, fout) ? 1u : 0u;
       chg += sweep_groups<NT, 32, 8>(a, B[1], B[2], lin, lout, smem_warp, majority, fin, fout);
       chg += sweep_groups<NT, 32, 4>(a, B[2], B[3], lin, lout, smem_warp, majority, fin, fout);
-      if (a.mode & kB3Half) chg += sweep_groups<NT, 16, 4>(a, B[3], B[4], lin, lout, smem_warp, majority, fin, fout);
+      if (a.mode & kB3Half) chg += sweep_threads<NT, 32, 2>(a, B[3], B[4], lin, lout, smem_warp, fin, fout);
       else chg += sweep_groups<NT, 32, 2>(a, B[3], B[4], lin, lout, smem_warp, majority, fin, fout);
       if (a.mode & kB4Threads) chg += sweep_threads<NT, 32>(a, B[4], B[5], lin, lout, smem_warp, fin, fout);
       else chg += sweep_groups<NT, 8, 4>(a, B[4], B[5], lin, lout, smem_warp, majority, fin, fout);
@@ -661,10 +672,14 @@ __global__ void __launch_bounds__(256) k_order_scatter(const int64_t* __restrict
   }
 }
 
+constexpr int kLargeNT = 768;
 struct Config {
-  int nt = 1024;   // threads per CTA
+  // threads per CTA: kLargeNT (what batch_threads = 1024 asks for: 1024 threads
+  // have 64 registers each and spill; 256 planted graphs, 20 steps: 28.4 ms with
+  // 1024 threads, 24.1 with 768, 25.4 with 512) or 512
+  int nt = kLargeNT;
   int tt = 32;     // degrees <= tt: a thread per vertex (8, 16 or 32)
-  int half = 1;    // degrees 33..64: 16-lane groups (else whole warps)
+  int half = 1;    // degrees 33..64: two threads each (else whole warps)
   unsigned long long barrier_ns = kBarrierLimitNs;  // grid-barrier wait limit
   int skip_cta = 0;  // failure tests: 1 + a CTA withholding its first arrival
   int blocks = 0;    // CTAs of the cooperative grid (0: as many as fit every SM)
@@ -769,7 +784,7 @@ int launch_k(glp_batch* b, const BatchArgs& a, size_t smem, cudaStream_t s, int 
 int launch_cfg(glp_batch* b, const Config& c, const BatchArgs& a, cudaStream_t s) {
   const size_t smem = std::max<size_t>((size_t)(c.nt / 32) * a.warp_words, 2 * (size_t)a.blk_cap) * sizeof(uint32_t);
   if (c.nt == 512) return launch_k<512>(b, a, smem, s, c.blocks);
-  if (c.nt == 1024) return launch_k<1024>(b, a, smem, s, c.blocks);
+  if (c.nt == kLargeNT) return launch_k<kLargeNT>(b, a, smem, s, c.blocks);
   set_error("no batch kernel for %d threads per block", c.nt);
   return GLP_EINVAL;
 }
@@ -799,10 +814,10 @@ BatchArgs make_args(glp_batch* b, const Config& c, int32_t niter) {
   for (int k = 0; k <= b->nclass; ++k) a.class_v[k] = b->class_v[k];
   a.mode = (c.tt >= 32 ? kB4Threads : 0u) | (c.tt >= 16 ? kB5Threads : 0u) | (c.half ? kB3Half : 0u);
   // a warp's 32 staged rows, or the tables of its groups (all alike)
-  static_assert(group_slots<32, 8>() == group_slots<32, 4>() && 2 * group_slots<16, 4>() == group_slots<32, 4>() &&
+  static_assert(group_slots<32, 8>() == group_slots<32, 4>() && group_slots<32, 2>() <= group_slots<32, 4>() &&
                     4 * group_slots<8, 4>() == group_slots<32, 4>() && 8 * group_slots<4, 4>() == group_slots<32, 4>(),
                 "one slice serves every group size");
-  a.warp_words = std::max<uint32_t>(32u * (uint32_t)c.tt, group_slots<32, 4>() * 3 / 2);
+  a.warp_words = std::max<uint32_t>(32u * (uint32_t)(c.half ? 32 : c.tt), group_slots<32, 4>() * 3 / 2);
   const int bdeg = max_degree_in(b, 256, kBatchMaxDegree);
   a.blk_cap = bdeg ? pow2_host(2u * (uint32_t)bdeg) : 0u;
   a.lab0 = b->d_lab[0];
@@ -861,7 +876,8 @@ Config config_from(const glp_batch* b, const glp_params* p) {
     if (p->tiny_max == 8 || p->tiny_max == 16 || p->tiny_max == 32) c.tt = p->tiny_max;
     if (p->mid_max == 32) c.half = 0;
     if (p->mid_max == 64) c.half = 1;
-    if (p->batch_threads == 512 || p->batch_threads == 1024) c.nt = p->batch_threads;
+    if (p->batch_threads == 512) c.nt = 512;
+    if (p->batch_threads == 1024) c.nt = kLargeNT;
     c.barrier_ns = p->barrier_limit_us > 0 ? 1000ull * (unsigned long long)p->barrier_limit_us : kBarrierLimitNs;
     c.skip_cta = p->fault_skip_cta > 0 ? p->fault_skip_cta : 0;
     c.blocks = p->batch_blocks > 0 ? p->batch_blocks : 0;
@@ -1234,7 +1250,7 @@ int glp_batch_tune(glp_batch* b, int32_t probe_iters, glp_params* best, float* t
     return GLP_EINVAL;
   }
   std::vector<Config> cands;
-  for (int nt : {512, 1024})
+  for (int nt : {512, kLargeNT})
     for (int tt : {8, 16, 32})
       for (int half : {0, 1}) cands.push_back(Config{nt, tt, half});
   if (ncand) *ncand = (int32_t)cands.size();
@@ -1282,7 +1298,7 @@ int glp_batch_tune(glp_batch* b, int32_t probe_iters, glp_params* best, float* t
     glp_params_default(best);
     best->tiny_max = best_c.tt;
     best->mid_max = best_c.half ? 64 : 32;
-    best->batch_threads = best_c.nt;
+    best->batch_threads = best_c.nt == kLargeNT ? 1024 : best_c.nt;
   }
   return GLP_OK;
 }

@@ -97,7 +97,8 @@ typedef struct glp_params {
                                      reported by glp_graph_check(); the
                                      stream must stay valid until the next
                                      call on the handle */
-  int32_t batch_threads;          /* glp_batch_run: threads per block, 512 or 1024 (0 = tuned / default) */
+  int32_t batch_threads;          /* glp_batch_run: threads per block, 512, or 1024 for the largest block the
+                                     kernel's registers allow (768) (0 = tuned / default) */
   int32_t barrier_limit_us;       /* glp_batch_run: how long a grid barrier of the persistent kernel
                                      waits before the run gives up with GLP_ETIMEOUT (0 = 5 s) */
   int32_t fault_skip_cta;         /* glp_batch_run, for tests of the failure path: 1 + the index of a
@@ -354,7 +355,7 @@ int glp_batch_info(const glp_batch* b, int64_t* n, int64_t* m, int32_t* max_degr
  * the largest iteration count, labels changed per iteration over the batch.  params (nullable; other
  * values = the tuned or default choice): tiny_max in {8,16,32} = largest
  * degree counted by one thread per vertex (above it, up to 32, lane groups);
- * mid_max 64 = degrees 33..64 by 16-lane groups, 32 = by whole warps;
+ * mid_max 64 = degrees 33..64 by two threads each, 32 = by whole warps;
  * batch_threads in {512,1024} = threads per block; use_graph = 1 captures the
  * run (counter resets, the persistent launch, a device-side label copy) in a
  * CUDA graph once and replays it while niter, the configuration, the stream
