@@ -320,20 +320,32 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     GLP_CUDA(cudaMemcpy(hub_off.data(), g->d_off, sizeof(int32_t) * hub_off.size(), cudaMemcpyDeviceToHost));
     build_host_plan(hub_off.data(), b[0], t, &hp);  // all of them are hubs
     for (int r = 0; r < kBigParts; ++r) p.big_part[r] = range_verts(b[kBigParts - 1 - r], b[kBigParts - r]);
+    p.big_low = range_verts(b[kBigParts - 1 - kBigLowParts + 1], b[kBigParts]);
     p.big = range_verts(b[0], b[kBigParts]);
     p.mid = range_verts(b[kBigParts], b[kBigParts + 1]);
     p.mb = range_verts(b[0], b[kBigParts + 1]);
     p.pair = range_verts(b[kBigParts + 5], b[kBigParts + 1]);
     p.mid_rest = range_verts(b[kBigParts], b[kBigParts + 5]);
     p.mb_rest = range_verts(b[0], b[kBigParts + 5]);
-    p.g32 = range_verts(b[kBigParts + 1], b[kBigParts + 2]);
-    p.g16 = range_verts(b[kBigParts + 2], b[kBigParts + 3]);
-    p.tiny = range_verts(b[kBigParts + 3], b[kBigParts + 4]);
+    p.merged = b[kBigParts + 4] <= kSmallGraph;
+    p.g32 = range_verts(b[kBigParts + 1], b[kBigParts + (p.merged ? 4 : 2)]);
+    if (!p.merged) {
+      p.g16 = range_verts(b[kBigParts + 2], b[kBigParts + 3]);
+      p.tiny = range_verts(b[kBigParts + 3], b[kBigParts + 4]);
+    }
     p.isolated = g->n - b[kBigParts + 4];
   } else {
     if ((rc = ensure_host_offsets(g))) return rc;
     build_host_plan(g->h_off.data(), g->n, t, &hp);
     p.isolated = hp.isolated;
+    p.merged = g->n - hp.isolated <= kSmallGraph;
+    if (p.merged) {
+      for (std::vector<int32_t>* v : {&hp.g16, &hp.tiny}) {
+        hp.g32.insert(hp.g32.end(), v->begin(), v->end());
+        v->clear();
+      }
+      std::sort(hp.g32.begin(), hp.g32.end());
+    }
     if ((rc = upload_verts(&p, hp.tiny, &p.tiny)) || (rc = upload_verts(&p, hp.g16, &p.g16)) ||
         (rc = upload_verts(&p, hp.g32, &p.g32)) || (rc = upload_verts(&p, hp.mid, &p.mid)) ||
         (rc = upload_verts(&p, hp.big, &p.big)) || (rc = upload_verts(&p, hp.mb, &p.mb)) ||
@@ -347,6 +359,15 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
         free_plan(&p);
         return rc;
       }
+    if (p.merged) {
+      std::vector<int32_t> low;
+      for (int r = 0; r < kBigLowParts; ++r) low.insert(low.end(), hp.big_part[r].begin(), hp.big_part[r].end());
+      std::sort(low.begin(), low.end());
+      if ((rc = upload_verts(&p, low, &p.big_low))) {
+        free_plan(&p);
+        return rc;
+      }
+    }
   }
   n_mid = p.mid.n;
   n_big = p.big.n;
@@ -362,7 +383,7 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
       (rc = zeroed(&p, std::max<size_t>((size_t)g->n, 1), &p.chg[0])) ||
       (rc = zeroed(&p, std::max<size_t>((size_t)g->n, 1), &p.chg[1])) ||
       (rc = zeroed(&p, std::max<size_t>((size_t)g->n, 1), &p.cyc_old)) ||
-      (rc = zeroed(&p, std::max<size_t>((size_t)g->n, 1), &p.cyc_stamp)) || (rc = zeroed(&p, 1, &p.cyc_mism))) {
+      (rc = zeroed(&p, std::max<size_t>((size_t)g->n, 1), &p.cyc_stamp)) || (rc = zeroed(&p, 2, &p.cyc_words))) {
     free_plan(&p);
     return rc;
   }
@@ -380,7 +401,8 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
   p.fmid.count = p.counts;
   p.fbig.count = p.counts + 1;
   p.fscreen.count = p.counts + 9;
-  p.front.tiny_max = t.tiny_max;
+  p.front.tiny_max = p.merged ? 0 : t.tiny_max;
+  p.front.g16_max = p.merged ? 0 : 16;
   p.front.mid_max = t.mid_max;
   p.front.big_max = t.big_max;
   for (int k = 0; k < 5; ++k) {
@@ -487,6 +509,17 @@ static int launch_small(const StepArgs& a, const TierWork& tw, const S& score, c
   return GLP_OK;
 }
 
+// The big tier's ranges up to 4096 in one launch (merged plans).
+template <bool W, class S>
+static int launch_big_merged(const StepArgs& a, const TierWork& tw, const S& score, cudaStream_t s) {
+  const unsigned grid = (unsigned)std::min<int64_t>(tw.all.n, device_sms() * 32);
+  constexpr bool k16 = !W && S::kPacked;
+  const size_t sm = k16 ? 12ull * 4096 : 4ull * 4096 * sizeof(uint32_t);
+  GLP_CUDA(raise_smem_limit((const void*)k_big<512, W, S, k16>, sm));
+  k_big<512, W, S, k16><<<grid, 512, sm, s>>>(a, tw, score);
+  return GLP_OK;
+}
+
 template <bool W, class S>
 int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_t* launches) {
   StepLaunch L = Lin;
@@ -502,9 +535,9 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
   if ((rc = mark_on(s, 8, 0))) return rc;  // whole-step start
   const bool modal = a.mode != nullptr;
   if (modal) {
-    GLP_CUDA(cudaMemsetAsync(p.counts, 0, 7 * sizeof(uint32_t), s));
-    k_step_mode<<<1, 1, 0, s>>>(L.prev_changed, a.n, a.n - (int32_t)p.isolated, L.allow_majority,
-                                L.allow_frontier, L.majority_pm, L.frontier_pm, p.d_mode);
+    k_step_begin<<<L.cycle.chg_prev ? (unsigned)device_sms() * 2 : 1u, 256, 0, s>>>(
+        L.prev_changed, a.n, a.n - (int32_t)p.isolated, L.allow_majority, L.allow_frontier, L.majority_pm,
+        L.frontier_pm, p.d_mode, p.counts, L.chg_n, L.cycle);
     ++*launches;
     if (L.allow_frontier && L.front.chg_in) {
       k_frontier_push<<<device_sms() * 16, 256, 0, s>>>(a, L.front);
@@ -521,7 +554,7 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
   };
   // fork: hubs on aux[0], the small tiers on aux[1], the rest here
   GLP_CUDA(cudaEventRecord(L.fork, s));
-  GLP_CUDA(cudaStreamWaitEvent(L.aux[0], L.fork, 0));
+  if (p.n_hubs) GLP_CUDA(cudaStreamWaitEvent(L.aux[0], L.fork, 0));
   GLP_CUDA(cudaStreamWaitEvent(L.aux[1], L.fork, 0));
   constexpr int kMidNT = 256, kBigNT = 256, kHubNT = 512, kBucketNT = 512;
   if (p.n_hubs) {
@@ -602,6 +635,12 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
       const Verts& vs = p.big_part[r];
       if (!vs.n) continue;
       const TierWork tw{vs, none, none, 1};
+      if (p.merged && kBigPartMax[r] <= 4096 && !L.big_staged) {
+        if ((rc = launch_big_merged<W>(a, TierWork{p.big_low, none, none, 1}, score, s))) return rc;
+        ++*launches;
+        while (r + 1 < kBigParts && kBigPartMax[r + 1] <= 4096) ++r;  // the launch covered them
+        continue;
+      }
       const size_t smr = 4ull * kBigPartMax[r] * sizeof(uint32_t);
       const unsigned grid = (unsigned)std::min<int64_t>(vs.n, kMaxGrid);
       if (k16 && r < kBigParts - 1) {
@@ -704,9 +743,11 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     ++*launches;
   }
   // join
-  GLP_CUDA(cudaEventRecord(L.join[0], L.aux[0]));
+  if (p.n_hubs) {
+    GLP_CUDA(cudaEventRecord(L.join[0], L.aux[0]));
+    GLP_CUDA(cudaStreamWaitEvent(s, L.join[0], 0));
+  }
   GLP_CUDA(cudaEventRecord(L.join[1], L.aux[1]));
-  GLP_CUDA(cudaStreamWaitEvent(s, L.join[0], 0));
   GLP_CUDA(cudaStreamWaitEvent(s, L.join[1], 0));
   if ((rc = mark_on(s, 8, 1))) return rc;  // whole-step stop
   GLP_CUDA(cudaGetLastError());
@@ -1038,6 +1079,7 @@ static int run_classic(RunCtx& c, int32_t niter) {
   if (track) {
     if ((rc = ensure_cycle_state(g))) return rc;
     for (int k = 0; k < 4; ++k) g->h_cycle[k] = 0u;
+    GLP_CUDA(cudaMemsetAsync(g->plan.cyc_words, 0, 2 * sizeof(uint32_t), c.s));
   }
   const uint32_t cyc_cap = (uint32_t)std::max<int64_t>(1024, g->n / 8);
   const unsigned cyc_grid = (unsigned)device_sms() * 4;
@@ -1061,7 +1103,6 @@ static int run_classic(RunCtx& c, int32_t niter) {
     a.bb = bb;
     // the change list's readers: the cycle check and the next step's frontier
     a.chg_cap = std::max(cyc_cap, (uint32_t)((uint64_t)g->n * c.frontier_pm / 1000) + 1u);
-    if (fr) GLP_CUDA(cudaMemsetAsync(p.counts + 7 + (it & 1), 0, sizeof(uint32_t), c.s));
     StepLaunch L = c.launch();
     L.prev_changed = it > 0 ? g->d_changed + it - 1 : nullptr;
     L.allow_majority = 1;
@@ -1073,29 +1114,25 @@ static int run_classic(RunCtx& c, int32_t niter) {
       L.front.chg_in = p.chg[(it - 1) & 1];
       L.front.chg_in_n = p.counts + 7 + ((it - 1) & 1);
     }
+    L.chg_n = fr ? p.counts + 7 + (it & 1) : nullptr;
     const uint32_t tag = ++g->cyc_tag;
-    if (track && it >= 1) {
-      // before the step overwrites them: L_{it-1} of the vertices step it-1 changed
-      GLP_CUDA(cudaMemsetAsync(p.cyc_mism, 0, sizeof(uint32_t), c.s));
-      k_cycle_save<<<cyc_grid, 256, 0, c.s>>>(p.chg[(it - 1) & 1], p.counts + 7 + ((it - 1) & 1), cyc_cap,
-                                             g->d_lab[(it + 1) & 1], p.cyc_old, p.cyc_stamp, tag, p.cyc_mism);
-      ++c.launches;
-    }
+    if (track && it >= 1)  // before the step overwrites them: L_{it-1} of the vertices step it-1 changed
+      L.cycle = CycleWatch{p.chg[(it - 1) & 1], p.counts + 7 + ((it - 1) & 1), cyc_cap, g->d_lab[(it + 1) & 1],
+                           p.cyc_old, p.cyc_stamp, tag, p.cyc_words};
     if (it == 0 && g->rows_sorted == 1) {
       if (c.timing) {  // first_step takes the step's events itself
         c.used--;
         c.ran.pop_back();
       }
+      if (fr) GLP_CUDA(cudaMemsetAsync(L.chg_n, 0, sizeof(uint32_t), c.s));
       if ((rc = first_step<W>(c, a))) return rc;
     } else if ((rc = launch_step<W>(L, a, ScoreClassic{}, &c.launches))) {
       return rc;
     }
     if (track && it >= 1) {
-      k_cycle_check<<<cyc_grid, 256, 0, c.s>>>(p.chg[it & 1], p.counts + 7 + (it & 1), p.counts + 7 + ((it - 1) & 1),
-                                              cyc_cap, g->d_lab[(it + 1) & 1], p.cyc_old, p.cyc_stamp, tag,
-                                              p.cyc_mism);
-      k_cycle_verdict<<<1, 1, 0, c.s>>>(p.cyc_mism, g->d_cycle + (it & 3));
-      c.launches += 2;
+      k_cycle_end<<<cyc_grid, 256, 0, c.s>>>(p.chg[it & 1], p.counts + 7 + (it & 1), g->d_lab[(it + 1) & 1], L.cycle,
+                                            g->d_cycle + (it & 3));
+      ++c.launches;
       GLP_CUDA(cudaGetLastError());
       GLP_CUDA(cudaEventRecord(g->cyc_ev[it % 3], c.s));
     }

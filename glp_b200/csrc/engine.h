@@ -36,7 +36,11 @@ constexpr int kMidCap = 512, kBigCap = 16384;
 // kBigCap-slot table (128 KB) and so cap big_max at kBigMaxWeighted.
 constexpr int kBigParts = 5;
 constexpr int kBigPartMax[kBigParts] = {1024, 2048, 4096, 8192, 24576};
+constexpr int kBigLowParts = 3;  // ranges up to 4096 (merged plans)
 constexpr int kBigPartThreads[kBigParts] = {256, 256, 512, 1024, 1024};
+// Graphs of at most this many non-isolated vertices run merged tiers: a step
+// of theirs is bound by its launches (see DevicePlan::merged).
+constexpr int64_t kSmallGraph = 1 << 18;
 constexpr int kBigMaxWeighted = 12288, kBigMaxUnweighted = 24576;
 static_assert(kBigCap == (int)kBig32Slots, "the engine sizes 32-bit big tables as k_big caps them");
 
@@ -75,7 +79,8 @@ struct DevicePlan {
   cudaStream_t setup = nullptr;  // stream of the set-up copies (the handle's)
   TierParams tiers;
   bool valid = false;
-  Verts tiny{}, g16{}, g32{}, mid{}, big{}, mb{}, pair{}, mid_rest{}, mb_rest{}, big_part[kBigParts]{};
+  Verts tiny{}, g16{}, g32{}, mid{}, big{}, mb{}, pair{}, mid_rest{}, mb_rest{},
+      big_low{}, big_part[kBigParts]{};
   FailList fmid{}, fbig{};
   FailList fscreen{};  // big-tier vertices a summary screen left to the exact kernel
   // list counters: [majority mid, majority big, frontier tiny, g16, g32, mid,
@@ -86,13 +91,16 @@ struct DevicePlan {
   Frontier front{};
   int32_t* d_mode = nullptr;
   // two-step cycle detection (classic, symmetric): labels before the last
-  // change, their step tags, and a mismatch word
+  // change, their step tags, and its words
   int32_t* cyc_old = nullptr;
   uint32_t* cyc_stamp = nullptr;
-  uint32_t* cyc_mism = nullptr;
+  uint32_t* cyc_words = nullptr;  // CycleWatch::words
   bool mid_c16 = true;  // mid counts fit 16 bits (unweighted, or small weight sums)
   int32_t n_hubs = 0, n_chunks = 0;
   int64_t isolated = 0;
+  // few vertices (kSmallGraph): the small tiers are one (g32) and the big tier's
+  // ranges up to 4096 one launch, since launches bound such a graph's steps
+  bool merged = false;
   bool sorted = false;  // degrees never increase along the ids: every tier is a range, isolated vertices last
   HubPlan hub{};
   BigBound bb{};  // count bounds of a contiguous big tier (n = 0: the tier is an id list)
@@ -108,7 +116,7 @@ struct StepLaunch {
   cudaEvent_t* ev;  // nullable: (start, stop) pairs for per-tier timing
   cudaStream_t aux[2];
   cudaEvent_t fork, join[2];
-  // step-mode inputs (k_step_mode): previous step's changed count (nullptr
+  // step-mode inputs (k_step_begin): previous step's changed count (nullptr
   // in the first step) and which shortcuts the method admits
   const unsigned long long* prev_changed = nullptr;
   int allow_majority = 0, allow_frontier = 0;
@@ -118,6 +126,8 @@ struct StepLaunch {
   uint32_t majority_pm = 500, frontier_pm = 50;  // step-mode thresholds (changes per 1000 vertices)
   bool mid_prefetch = true;  // k_mid loads the next vertex's first batch while counting
   bool big_staged = false;   // k_big_staged for the first big range of full-count steps
+  CycleWatch cycle{};       // two-step cycle detection: what k_step_begin keeps
+  uint32_t* chg_n = nullptr;  // this step's changed-list counter, cleared by k_step_begin
   // k_hub_bound may decide hubs from their earlier counts: classic steps,
   // whose gathered labels are the current labels (not SLPA's spoken ones)
   bool hub_bound = false;

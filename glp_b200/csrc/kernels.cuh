@@ -60,7 +60,7 @@ struct StepArgs {
   int32_t* lout;
   unsigned long long* changed;
   uint32_t* err;
-  // this step's mode, set on the device by k_step_mode (nullptr: full)
+  // this step's mode, set on the device by k_step_begin (nullptr: full)
   const int32_t* mode;
   int32_t n;
   // vertices whose label changed this step are appended here (nullable); a
@@ -156,8 +156,9 @@ __device__ __forceinline__ bool use_majority(const StepArgs& a) { return step_mo
 // of the n_active non-isolated vertices changed (their neighbourhoods hold
 // few distinct labels); 0 = score at every insert, the lookup issued before
 // the insert so that its latency overlaps the hashing.
-__global__ void k_step_mode(const unsigned long long* prev_changed, int32_t n, int32_t n_active, int allow_majority,
-                            int allow_frontier, uint32_t majority_pm, uint32_t frontier_pm, int32_t* mode) {
+__device__ __forceinline__ void step_mode_of(const unsigned long long* prev_changed, int32_t n, int32_t n_active,
+                                             int allow_majority, int allow_frontier, uint32_t majority_pm,
+                                             uint32_t frontier_pm, int32_t* mode) {
   int32_t m = kModeFull, scan = 0;
   if (prev_changed) {
     const unsigned long long c = *prev_changed;
@@ -1467,45 +1468,68 @@ __global__ void k_hub_finalize(StepArgs a, HubPlan hp, const uint8_t* seeds) {
 // labels for ever.  Once a step ends in that cycle every later labeling is
 // known exactly, so a run can stop there.  With S_t the vertices step t
 // changes (L_{t+1}(v) != L_t(v)), L_{t+1} = L_{t-1} holds iff S_t = S_{t-1}
-// and every v in S_t returns to L_{t-1}(v).  k_cycle_save keeps L_{t-1}(v)
-// for v in S_{t-1} before step t overwrites it; k_cycle_check compares after
-// the step; k_cycle_verdict publishes the answer to the host.  The lists are
+// and every v in S_t returns to L_{t-1}(v).  k_step_begin keeps L_{t-1}(v)
+// for v in S_{t-1} before step t overwrites it; k_cycle_end compares after the
+// step and publishes the answer to the host.  The lists are
 // walked only while they are short (at most `cap` entries); a longer list
 // marks the step as not cyclic.
-__global__ void k_cycle_save(const int32_t* __restrict__ chg_prev, const uint32_t* n_prev, uint32_t cap,
-                             const int32_t* __restrict__ lab_prev2, int32_t* __restrict__ old,
-                             uint32_t* __restrict__ stamp, uint32_t tag, uint32_t* mism) {
-  const uint32_t c = *n_prev;
-  if (c > cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(mism, 1u);
+struct CycleWatch {
+  const int32_t* chg_prev = nullptr;  // vertices the previous step changed (nullptr: not watched)
+  const uint32_t* n_prev = nullptr;
+  uint32_t cap = 0;
+  const int32_t* lab_prev2 = nullptr;  // labels before the previous step, which this step overwrites
+  int32_t* old = nullptr;
+  uint32_t* stamp = nullptr;
+  uint32_t tag = 0;
+  uint32_t* words = nullptr;  // [0] mismatch, [1] blocks of k_cycle_end that are done; both 0 between steps
+};
+
+// Everything a step does before its tiers, in one launch: the step's counters
+// are cleared and its mode chosen (thread 0 of block 0), and the labels the
+// cycle check will need are kept.  A memset or a
+// one-thread kernel of its own costs a small graph's step as much as a tier.
+__global__ void k_step_begin(const unsigned long long* prev_changed, int32_t n, int32_t n_active, int allow_majority,
+                             int allow_frontier, uint32_t majority_pm, uint32_t frontier_pm, int32_t* mode,
+                             uint32_t* counts, uint32_t* chg_n, CycleWatch w) {
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < 7) counts[threadIdx.x] = 0u;
+    if (threadIdx.x == 7 && chg_n) *chg_n = 0u;
+    if (threadIdx.x == 0)
+      step_mode_of(prev_changed, n, n_active, allow_majority, allow_frontier, majority_pm, frontier_pm, mode);
+  }
+  if (!w.chg_prev) return;
+  const uint32_t c = *w.n_prev;
+  if (c > w.cap) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) w.words[0] = 1u;
     return;
   }
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c; i += gridDim.x * blockDim.x) {
-    const int32_t v = chg_prev[i];
-    old[v] = lab_prev2[v];
-    stamp[v] = tag;
+    const int32_t v = w.chg_prev[i];
+    w.old[v] = w.lab_prev2[v];
+    w.stamp[v] = w.tag;
   }
 }
 
-__global__ void k_cycle_check(const int32_t* __restrict__ chg, const uint32_t* n_now, const uint32_t* n_prev,
-                              uint32_t cap, const int32_t* __restrict__ lab_next, const int32_t* __restrict__ old,
-                              const uint32_t* __restrict__ stamp, uint32_t tag, uint32_t* mism) {
+// Compares after the step; the last block to finish publishes the verdict
+// (flag: host-mapped word; 1 = the step ended in a two-step cycle) and clears
+// the words for the next step.
+__global__ void k_cycle_end(const int32_t* __restrict__ chg, const uint32_t* n_now,
+                            const int32_t* __restrict__ lab_next, CycleWatch w, volatile uint32_t* flag) {
   const uint32_t c = *n_now;
-  if (c != *n_prev || c > cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(mism, 1u);
-    return;
-  }
-  bool bad = false;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c; i += gridDim.x * blockDim.x) {
-    const int32_t v = chg[i];
-    bad |= stamp[v] != tag || lab_next[v] != old[v];
-  }
-  if (__any_sync(kFull, bad) && (threadIdx.x & 31) == 0) atomicOr(mism, 1u);
-}
-
-// flag: host-mapped word; 1 = the step ended in a two-step cycle.
-__global__ void k_cycle_verdict(const uint32_t* mism, volatile uint32_t* flag) {
-  *flag = *mism == 0u ? 1u : 0u;
+  bool bad = c != *w.n_prev || c > w.cap;
+  if (!bad)
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c; i += gridDim.x * blockDim.x) {
+      const int32_t v = chg[i];
+      bad |= w.stamp[v] != w.tag || lab_next[v] != w.old[v];
+    }
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x != 0) return;
+  if (bad) atomicOr(w.words, 1u);
+  __threadfence();
+  if (atomicAdd(w.words + 1, 1u) + 1u != gridDim.x) return;
+  __threadfence();
+  *flag = atomicExch(w.words, 0u) == 0u ? 1u : 0u;
+  w.words[1] = 0u;
   __threadfence_system();
 }
 
@@ -1657,7 +1681,7 @@ struct Frontier {
   uint32_t epoch;          // this step's mark (unique per step of the handle)
   const int32_t* chg_in;   // vertices changed in the previous step
   const uint32_t* chg_in_n;
-  int32_t tiny_max, mid_max, big_max;
+  int32_t tiny_max, g16_max, mid_max, big_max;
   FailList tier[5];        // frontier members of tiny, g16, g32, mid, big
 };
 
@@ -1731,7 +1755,7 @@ __global__ void __launch_bounds__(256) k_frontier_list(StepArgs a, Frontier f, i
       const int64_t v = v0 + q * 256 + threadIdx.x;
       if (tier[q] == 0) {
         const int32_t d = a.off[v + 1] - a.off[v];
-        tier[q] = d <= f.tiny_max ? 0 : d <= 16 ? 1 : d <= 32 ? 2 : d <= f.mid_max ? 3 : d <= f.big_max ? 4 : -1;
+        tier[q] = d <= f.tiny_max ? 0 : d <= f.g16_max ? 1 : d <= 32 ? 2 : d <= f.mid_max ? 3 : d <= f.big_max ? 4 : -1;
       }
     }
 #pragma unroll

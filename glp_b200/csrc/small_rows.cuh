@@ -104,7 +104,9 @@ __device__ __forceinline__ int32_t small_row_best(const S& score, const uint32_t
   } else if constexpr (R == 16) {
     return dmax <= 12 ? small_best<12, R, W, S, K>(score, slab, t, d) : small_best<16, R, W, S, K>(score, slab, t, d);
   } else {
-    return dmax <= 20   ? small_best<20, R, W, S, K>(score, slab, t, d)
+    return dmax <= 8    ? small_best<8, R, W, S, K>(score, slab, t, d)  // a small graph's merged tiers
+           : dmax <= 16 ? small_best<16, R, W, S, K>(score, slab, t, d)
+           : dmax <= 20 ? small_best<20, R, W, S, K>(score, slab, t, d)
            : dmax <= 24 ? small_best<24, R, W, S, K>(score, slab, t, d)
            : dmax <= 28 ? small_best<28, R, W, S, K>(score, slab, t, d)
                         : small_best<32, R, W, S, K>(score, slab, t, d);
