@@ -266,20 +266,42 @@ __device__ __forceinline__ bool group_vertex(const BatchArgs& a, int32_t v, cons
   return gl == 0 && l != own;
 }
 
+// Deals a step's warp tasks round robin over the grid's warps, from one sweep
+// to the next without a break: a warp that got no task in a sweep's last round
+// starts the next sweep, so small buckets do not cost a round of latency each
+// (10 graphs of 216 thousand vertices, 11 steps: 475 -> 335 us).  Neighbouring
+// tasks go to the warps of one SM, whose L1 then holds their graph's labels
+// (spread over the SMs, 256 graphs took 32.9 ms instead of 24), but over the
+// SMs in a batch of at most four rounds, which would leave SMs without work.
+struct Turns {
+  uint32_t warps, mine, next = 0;  // next: the warp whose turn it is
+  template <int NT>
+  static __device__ __forceinline__ Turns of(int64_t n) {
+    const uint32_t w = threadIdx.x >> 5, warps = gridDim.x * (NT / 32);
+    return Turns{warps, n > 4 * 32ll * warps ? blockIdx.x * (NT / 32) + w : w * gridDim.x + blockIdx.x};
+  }
+  // This warp's first task among those of n vertices, V to a task.
+  template <int V>
+  __device__ __forceinline__ int64_t first(int64_t n) {
+    const uint32_t f = mine >= next ? mine - next : mine + warps - next;
+    next = (next + (uint32_t)((n + V - 1) / V)) % warps;
+    return f;
+  }
+};
+
 // Sweep order[lo, hi) with groups of G lanes; smem_warp: this warp's slice.
 template <int NT, int G, int L>
 __device__ __forceinline__ uint32_t sweep_groups(const BatchArgs& a, int64_t lo, int64_t hi,
                                                  const int32_t* __restrict__ lin, int32_t* __restrict__ lout,
                                                  uint32_t* smem_warp, bool majority, const uint8_t* fin,
-                                                 uint8_t* fout) {
+                                                 uint8_t* fout, Turns& turns) {
   constexpr int kGroups = 32 / G;
   constexpr uint32_t kSlots = group_slots<G, L>();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int grp = lane / G;
   uint32_t* keys = smem_warp + (size_t)grp * (kSlots + kSlots / 2);
-  const int64_t nw = (int64_t)gridDim.x * (NT / 32);
   uint32_t chg = 0;
-  for (int64_t i0 = lo + ((int64_t)blockIdx.x * (NT / 32) + warp) * kGroups; i0 < hi; i0 += nw * kGroups) {
+  for (int64_t i0 = lo + turns.first<kGroups>(hi - lo) * kGroups; i0 < hi; i0 += (int64_t)turns.warps * kGroups) {
     const int64_t i = i0 + grp;
     const int32_t v = i < hi ? a.order[i] : -1;
     chg += group_vertex<G, L>(a, v, lin, lout, keys, majority, fin, fout) ? 1u : 0u;
@@ -363,15 +385,16 @@ __device__ __forceinline__ bool block_vertex(const BatchArgs& a, int32_t v, cons
 // its labels in registers and reads the counts off the runs.  A thread loading
 // its own row, 32 sectors a load, and sorting with a bitonic network, and
 // 16-lane groups with a count table for degrees 33..64, took 38.7 ms for 256
-// planted graphs and 20 steps (4.8 G entries); these sweeps take 24.1.
+// planted graphs and 20 steps (4.8 G entries); these sweeps take 23.7.
 template <int NT, int R, int L = 1>
 __device__ __forceinline__ uint32_t sweep_threads(const BatchArgs& a, int64_t lo, int64_t hi,
                                                   const int32_t* __restrict__ lin, int32_t* __restrict__ lout,
-                                                  uint32_t* slab, const uint8_t* fin, uint8_t* fout) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane >> 3, sub = lane & (L - 1);
+                                                  uint32_t* slab, const uint8_t* fin, uint8_t* fout,
+                                                  Turns& turns) {
+  constexpr int V = 32 / L;
+  const int lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & (L - 1);
   uint32_t chg = 0;
-  for (int64_t i0 = lo + ((int64_t)blockIdx.x * NT + warp * 32) / L; i0 < hi;
-       i0 += (int64_t)gridDim.x * NT / L) {  // warp-uniform
+  for (int64_t i0 = lo + turns.first<V>(hi - lo) * V; i0 < hi; i0 += (int64_t)turns.warps * V) {  // warp-uniform
     int32_t v = -1, own = 0, d = 0;
     int64_t b = 0;
     if (i0 + lane / L < hi) {
@@ -521,20 +544,21 @@ __global__ void __launch_bounds__(NT) k_batch(BatchArgs a) {
                                                                                  : nullptr;
     uint8_t* fout = (it & 1) ? a.chg1 : a.chg0;
     uint32_t chg = 0;
+    Turns turns = Turns::of<NT>(a.n);
     for (int c = 0; c < a.nclass; ++c) {
       if (it >= a.class_niter[c]) continue;  // this class has finished
       const int64_t* B = a.bstart[c];
       for (int64_t i = B[0] + blockIdx.x; i < B[1]; i += gridDim.x)
         chg += block_vertex<NT>(a, a.order[i], lin, lout, smem, red, fin, fout) ? 1u : 0u;
-      chg += sweep_groups<NT, 32, 8>(a, B[1], B[2], lin, lout, smem_warp, majority, fin, fout);
-      chg += sweep_groups<NT, 32, 4>(a, B[2], B[3], lin, lout, smem_warp, majority, fin, fout);
-      if (a.mode & kB3Half) chg += sweep_threads<NT, 32, 2>(a, B[3], B[4], lin, lout, smem_warp, fin, fout);
-      else chg += sweep_groups<NT, 32, 2>(a, B[3], B[4], lin, lout, smem_warp, majority, fin, fout);
-      if (a.mode & kB4Threads) chg += sweep_threads<NT, 32>(a, B[4], B[5], lin, lout, smem_warp, fin, fout);
-      else chg += sweep_groups<NT, 8, 4>(a, B[4], B[5], lin, lout, smem_warp, majority, fin, fout);
-      if (a.mode & kB5Threads) chg += sweep_threads<NT, 16>(a, B[5], B[6], lin, lout, smem_warp, fin, fout);
-      else chg += sweep_groups<NT, 4, 4>(a, B[5], B[6], lin, lout, smem_warp, majority, fin, fout);
-      chg += sweep_threads<NT, 8>(a, B[6], B[7], lin, lout, smem_warp, fin, fout);
+      chg += sweep_groups<NT, 32, 8>(a, B[1], B[2], lin, lout, smem_warp, majority, fin, fout, turns);
+      chg += sweep_groups<NT, 32, 4>(a, B[2], B[3], lin, lout, smem_warp, majority, fin, fout, turns);
+      if (a.mode & kB3Half) chg += sweep_threads<NT, 32, 2>(a, B[3], B[4], lin, lout, smem_warp, fin, fout, turns);
+      else chg += sweep_groups<NT, 32, 2>(a, B[3], B[4], lin, lout, smem_warp, majority, fin, fout, turns);
+      if (a.mode & kB4Threads) chg += sweep_threads<NT, 32>(a, B[4], B[5], lin, lout, smem_warp, fin, fout, turns);
+      else chg += sweep_groups<NT, 8, 4>(a, B[4], B[5], lin, lout, smem_warp, majority, fin, fout, turns);
+      if (a.mode & kB5Threads) chg += sweep_threads<NT, 16>(a, B[5], B[6], lin, lout, smem_warp, fin, fout, turns);
+      else chg += sweep_groups<NT, 4, 4>(a, B[5], B[6], lin, lout, smem_warp, majority, fin, fout, turns);
+      chg += sweep_threads<NT, 8>(a, B[6], B[7], lin, lout, smem_warp, fin, fout, turns);
     }
     block_count_add<NT>(a.changed + it, chg, red_u);
     if (it + 1 < a.niter && !grid_barrier(a.bar, ++phase * gridDim.x, a.err, a.barrier_ns)) return;
@@ -672,11 +696,11 @@ __global__ void __launch_bounds__(256) k_order_scatter(const int64_t* __restrict
   }
 }
 
-constexpr int kLargeNT = 768;
+constexpr int kLargeNT = 640;
 struct Config {
   // threads per CTA: kLargeNT (what batch_threads = 1024 asks for: 1024 threads
   // have 64 registers each and spill; 256 planted graphs, 20 steps: 28.4 ms with
-  // 1024 threads, 24.1 with 768, 25.4 with 512) or 512
+  // 1024 threads, 27.0 with 768, 23.7 with 640, 25.4 with 512) or 512
   int nt = kLargeNT;
   int tt = 32;     // degrees <= tt: a thread per vertex (8, 16 or 32)
   int half = 1;    // degrees 33..64: two threads each (else whole warps)

@@ -98,7 +98,7 @@ typedef struct glp_params {
                                      stream must stay valid until the next
                                      call on the handle */
   int32_t batch_threads;          /* glp_batch_run: threads per block, 512, or 1024 for the largest block the
-                                     kernel's registers allow (768) (0 = tuned / default) */
+                                     kernel's registers allow (640) (0 = tuned / default) */
   int32_t barrier_limit_us;       /* glp_batch_run: how long a grid barrier of the persistent kernel
                                      waits before the run gives up with GLP_ETIMEOUT (0 = 5 s) */
   int32_t fault_skip_cta;         /* glp_batch_run, for tests of the failure path: 1 + the index of a
