@@ -560,7 +560,7 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
   if (p.n_hubs) {
     const size_t sm = 2ull * kHubTable * sizeof(uint32_t);
     const size_t sm_hist = (size_t)p.hub.max_nb * sizeof(uint32_t);
-    if ((rc = allow_smem(k_hub_bucket<kBucketNT, W, S>, sm)) || (rc = allow_smem(k_hub_gather<kHubNT, W>, sm_hist)) ||
+    if ((rc = allow_smem(k_hub_bucket<kBucketNT, W, S>, sm)) || (rc = allow_smem(k_hub_gather<kHubNT, W, S>, sm_hist)) ||
         (rc = allow_smem(k_hub_scatter<kHubNT, W>, 2 * sm_hist)))
       return rc;
     if ((rc = mark_on(L.aux[0], 5, 0))) return rc;
@@ -573,7 +573,7 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     }
     k_hub_decide<<<hgrid, 256, 0, L.aux[0]>>>(a, p.hub);
     GLP_CUDA(cudaMemsetAsync(p.hub.bcnt, 0, sizeof(uint32_t) * p.hub.nitems, L.aux[0]));
-    k_hub_gather<kHubNT, W><<<grid, kHubNT, sm_hist, L.aux[0]>>>(a, p.hub, p.n_chunks);
+    k_hub_gather<kHubNT, W, S><<<grid, kHubNT, sm_hist, L.aux[0]>>>(a, p.hub, p.n_chunks, score);
     k_hub_offsets<<<hgrid, 256, 0, L.aux[0]>>>(p.hub);
     k_hub_scatter<kHubNT, W><<<grid, kHubNT, 2 * sm_hist, L.aux[0]>>>(a, p.hub, p.n_chunks);
     k_hub_bucket<kBucketNT, W, S><<<(unsigned)std::min<int64_t>(p.hub.nitems, device_sms() * 8), kBucketNT, sm, L.aux[0]>>>(
@@ -1216,7 +1216,7 @@ static int run_layered(RunCtx& c, const glp_params& p, int32_t niter) {
           k_label_volumes<<<lv_grid, 256, 0, c.s>>>(lin, vol_r, g->n, g->d_lv);
           ++c.launches;
         }
-        rc = launch_step<W>(L, a, ScoreLayered32{vol_r, p.dstar[layer], g->d_lv}, &c.launches);
+        rc = launch_step<W>(L, a, ScoreLayered32{vol_r, p.dstar[layer], g->d_lv, it > 0 && g->rows_sorted == 1}, &c.launches);
       } else {
         rc = launch_step<W>(L, a, ScoreLayered{vol_r, (int64_t)p.dstar[layer]}, &c.launches);
       }

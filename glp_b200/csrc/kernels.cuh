@@ -292,6 +292,10 @@ struct ScoreLayered32 {
   const int32_t* vol;
   int32_t dstar;
   const int2* lv;  // [n] (label of v, vol[label of v]); .x equals lin[v]
+  // vol counts the holders of each label among this step's input and no row
+  // lists a neighbour twice: a label of volume 1 occurs once in a row, so its
+  // count is its entry's weight and needs no table (ChunkQueue)
+  bool single;
   __device__ __forceinline__ void load(const StepArgs&, int32_t c, int32_t& lab, int32_t& vl) const {
     const int2 x = __ldg(lv + c);
     lab = x.x;
@@ -563,6 +567,56 @@ __device__ __forceinline__ void count_chunk(bool has, int32_t lab, uint32_t wt, 
   }
 }
 
+// The entries of a warp's row part that need the count table, for scores with
+// `single`: labels of volume 1 are scored where they are read, and the others
+// wait in a ring of 64 until 32 of them fill a chunk.  On R-MAT graphs 42 to
+// 85 % of the entries of a layered step have such labels (most vertices change
+// to a label of their own neighbourhood every step), and a chunk of the table
+// costs the same however few of its lanes have an entry.
+struct ChunkRing {
+  int2 lv[64];
+  uint32_t w[64];
+};
+template <bool W>
+struct ChunkQueue {
+  ChunkRing* ring;
+  uint32_t head = 0, fill = 0;  // warp-uniform
+  __device__ __forceinline__ explicit ChunkQueue(ChunkRing* r) : ring(r) {}
+  // Counts the first `n` waiting entries; every lane takes part.
+  template <class S, class Ins, class B>
+  __device__ __forceinline__ void count(uint32_t n, const S& score, const Ins& insert, B& best, bool& fail, bool scan,
+                                        bool merge) {
+    __syncwarp();
+    const uint32_t lane = threadIdx.x & 31, at = (head + lane) & 63u;
+    const bool has = lane < n;
+    const int2 e = has ? ring->lv[at] : make_int2(-1, 0);
+    const uint32_t wt = W && has ? ring->w[at] : (has ? 1u : 0u);
+    count_chunk<W, true>(has, e.x, wt, score, insert, best, fail, scan, e.y, merge);
+    head = (head + n) & 63u;
+    fill -= n;
+    __syncwarp();  // the words may be written again
+  }
+  template <class S, class Ins, class B>
+  __device__ __forceinline__ void add(bool has, int32_t lab, uint32_t wt, int32_t vl, const S& score,
+                                      const Ins& insert, B& best, bool& fail, bool scan, bool merge) {
+    const bool alone = has && vl == 1;
+    if (alone) offer(best, score, W ? wt : 1u, 1, lab);
+    const uint32_t m = __ballot_sync(kFull, has && !alone);
+    if (has && !alone) {
+      const uint32_t at = (head + fill + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))) & 63u;
+      ring->lv[at] = make_int2(lab, vl);
+      if (W) ring->w[at] = wt;
+    }
+    fill += __popc(m);
+    if (fill >= 32) count(32, score, insert, best, fail, scan, merge);
+  }
+  template <class S, class Ins, class B>
+  __device__ __forceinline__ void finish(const S& score, const Ins& insert, B& best, bool& fail, bool scan,
+                                         bool merge) {
+    if (fill) count(fill, score, insert, best, fail, scan, merge);
+  }
+};
+
 // The best (score, label) over the occupied slots of a finished table, slots
 // t, t+stride, ... of it (scores with kScan).
 // Eight slots a round (four in kernels held to 40 registers), their volume
@@ -692,6 +746,7 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
   __shared__ __align__(16) uint32_t skeys[NW][CAP];
   __shared__ __align__(16) uint32_t svals[NW][C16 ? CAP / 2 : CAP];
   __shared__ int32_t cbuf[NW][32];  // changed vertices not yet listed
+  __shared__ ChunkRing rings[S::kLV ? NW : 1];
   uint32_t ncb = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int32_t mode = step_mode(a);
@@ -769,6 +824,7 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
       return CF ? table_claim_insert<C16>(kk, vv, cap - 1, key, k, cap)
                 : table_insert_bounded<C16>(kk, vv, cap - 1, key, k, cap, nullptr, nullptr);
     };
+    ChunkQueue<W> queue(&rings[S::kLV ? warp : 0]);
     for (int32_t j0 = b; j0 < e; j0 += 128) {
       int32_t lab[4], vl[4];
       uint32_t wt[4];
@@ -782,11 +838,20 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
       } else {
         load_batch(j0, e, lab, wt, vl);
       }
+      if constexpr (S::kLV) {
+        if (score.single) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (j0 + 32 * q < e) queue.add(lab[q] >= 0, lab[q], wt[q], vl[q], score, ins, best, fail, scan, merge);
+          continue;
+        }
+      }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         if (j0 + 32 * q < e)
           count_chunk<W, S::kLV>(lab[q] >= 0, lab[q], wt[q], score, ins, best, fail, scan, vl[q], merge);
     }
+    if constexpr (S::kLV) queue.finish(score, ins, best, fail, scan, merge);
     if (fail) atomicOr(a.err, kErrProbe);
     if (scan) {
       __syncwarp();
@@ -854,6 +919,7 @@ __global__ void __launch_bounds__(NT, (!W ? ((NT == 1024 && S::kPacked) ? 2048 :
   const bool scan = S::kScan && scan_scores(a);
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ int32_t cbuf[64];  // changed vertices not yet listed (thread 0's)
+  __shared__ ChunkRing rings[S::kLV ? NT / 32 : 1];
   uint32_t ncb = 0;
   __shared__ Best red[32];
   // packed scores: one slot per vertex parity, so thread 0 can read vertex
@@ -968,6 +1034,7 @@ __global__ void __launch_bounds__(NT, (!W ? ((NT == 1024 && S::kPacked) ? 2048 :
     // degree-1 neighbours) fills many lanes of a chunk: without it those
     // lanes' adds to one slot serialise
     const bool merge = !CF || mode != kModeFull || (e - b) > kMergeDegree || S::kKeep;
+    ChunkQueue<W> queue(&rings[S::kLV ? warp : 0]);
     for (int32_t j0 = b + warp * 32; j0 < e; j0 += 4 * NT) {
       int32_t lab[4], vl[4];
       uint32_t wt[4];
@@ -980,11 +1047,20 @@ __global__ void __launch_bounds__(NT, (!W ? ((NT == 1024 && S::kPacked) ? 2048 :
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         if (lab[q] >= 0) score.load(a, lab[q], lab[q], vl[q]);
+      if constexpr (S::kLV) {
+        if (score.single) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (j0 + q * NT < e) queue.add(lab[q] >= 0, lab[q], wt[q], vl[q], score, ins, best, fail, scan, merge);
+          continue;
+        }
+      }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         if (j0 + q * NT < e)
           count_chunk<W, S::kLV>(lab[q] >= 0, lab[q], wt[q], score, ins, best, fail, scan, vl[q], merge);
     }
+    if constexpr (S::kLV) queue.finish(score, ins, best, fail, scan, merge);
     if (fail) atomicOr(a.err, kErrProbe);
     if (scan) {  // block-uniform
       __syncthreads();
@@ -1295,9 +1371,11 @@ __global__ void k_hub_decide(StepArgs a, HubPlan hp) {
 }
 
 // Gathers the labels of undecided hubs and counts them per bucket
-// (block-local histogram, one global add per nonzero bucket).
-template <int NT, bool W>
-__global__ void __launch_bounds__(NT) k_hub_gather(StepArgs a, HubPlan hp, int32_t nchunks) {
+// (block-local histogram, one global add per nonzero bucket).  An entry without
+// a label (seeded LP) is -1 and in no bucket; so is one whose label needs no
+// table (ScoreLayered32::single), which goes to the hub's best at once.
+template <int NT, bool W, class S>
+__global__ void __launch_bounds__(NT) k_hub_gather(StepArgs a, HubPlan hp, int32_t nchunks, S score) {
   extern __shared__ uint32_t hist[];  // [max_nb]
   for (int32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
     const int32_t h = hp.chunk_hub[c];
@@ -1307,6 +1385,7 @@ __global__ void __launch_bounds__(NT) k_hub_gather(StepArgs a, HubPlan hp, int32
     const int64_t base = hp.hub_lbase[h] - a.off[hp.hub_v[h]];
     for (uint32_t b = threadIdx.x; b < nb; b += NT) hist[b] = 0;
     __syncthreads();
+    Best alone = best_none();
     for (int32_t j0 = cb + threadIdx.x; j0 < ce; j0 += 4 * NT) {
       int32_t col[4];
 #pragma unroll
@@ -1315,10 +1394,31 @@ __global__ void __launch_bounds__(NT) k_hub_gather(StepArgs a, HubPlan hp, int32
       for (int q = 0; q < 4; ++q) {
         if (col[q] < 0) continue;
         const int32_t j = j0 + q * NT;
-        const int32_t l = ld_label(a.lin + col[q]);
+        int32_t l = -1, vl = 0;
+        const int32_t w = W ? ld_stream(a.w + j) : 1;
+        if constexpr (S::kLV) {
+          if (score.single) {
+            score.load(a, col[q], l, vl);
+            if (vl == 1) {
+              const Best x{score.from_vol((uint32_t)w, 1), l};
+              if (better(x, alone)) alone = x;
+              l = -1;
+            }
+          } else {
+            l = ld_label(a.lin + col[q]);
+          }
+        } else {
+          l = ld_label(a.lin + col[q]);
+        }
         hp.hlab[base + j] = l;
-        if (W) hp.hw[base + j] = ld_stream(a.w + j);
-        atomicAdd(hist + (nb > 1 ? hub_bucket_of((uint32_t)l + 1u, nb) : 0u), 1u);
+        if (W) hp.hw[base + j] = w;
+        if (l >= 0) atomicAdd(hist + (nb > 1 ? hub_bucket_of((uint32_t)l + 1u, nb) : 0u), 1u);
+      }
+    }
+    if constexpr (S::kLV) {
+      if (score.single) {
+        alone = group_max<32>(alone);
+        if ((threadIdx.x & 31) == 0 && alone.l >= 0) atomicMax(hp.hub_best + h, pack_best(alone, a.err));
       }
     }
     __syncthreads();
@@ -1362,13 +1462,14 @@ __global__ void __launch_bounds__(NT) k_hub_scatter(StepArgs a, HubPlan hp, int3
     __syncthreads();
     for (int32_t j = cb + threadIdx.x; j < ce; j += NT) {
       const int32_t l = hp.hlab[base + j];
-      atomicAdd(cnt + (nb > 1 ? hub_bucket_of((uint32_t)l + 1u, nb) : 0u), 1u);
+      if (l >= 0) atomicAdd(cnt + (nb > 1 ? hub_bucket_of((uint32_t)l + 1u, nb) : 0u), 1u);
     }
     __syncthreads();
     for (uint32_t b = threadIdx.x; b < nb; b += NT) cur[b] = cnt[b] ? atomicAdd(hp.bcur + item0 + b, cnt[b]) : 0u;
     __syncthreads();
     for (int32_t j = cb + threadIdx.x; j < ce; j += NT) {
       const int32_t l = hp.hlab[base + j];
+      if (l < 0) continue;
       const uint32_t b = nb > 1 ? hub_bucket_of((uint32_t)l + 1u, nb) : 0u;
       const uint32_t pos = atomicAdd(cur + b, 1u);
       hp.hsort[lb + pos] = l;
