@@ -320,6 +320,7 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     GLP_CUDA(cudaMemcpy(hub_off.data(), g->d_off, sizeof(int32_t) * hub_off.size(), cudaMemcpyDeviceToHost));
     build_host_plan(hub_off.data(), b[0], t, &hp);  // all of them are hubs
     for (int r = 0; r < kBigParts; ++r) p.big_part[r] = range_verts(b[kBigParts - 1 - r], b[kBigParts - r]);
+    p.big_first = range_verts(b[kBigParts - 2], b[kBigParts]);
     p.big_low = range_verts(b[kBigParts - 1 - kBigLowParts + 1], b[kBigParts]);
     p.big = range_verts(b[0], b[kBigParts]);
     p.mid = range_verts(b[kBigParts], b[kBigParts + 1]);
@@ -359,6 +360,13 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
         free_plan(&p);
         return rc;
       }
+    std::vector<int32_t> first = hp.big_part[0];
+    first.insert(first.end(), hp.big_part[1].begin(), hp.big_part[1].end());
+    std::sort(first.begin(), first.end());
+    if ((rc = upload_verts(&p, first, &p.big_first))) {
+      free_plan(&p);
+      return rc;
+    }
     if (p.merged) {
       std::vector<int32_t> low;
       for (int r = 0; r < kBigLowParts; ++r) low.insert(low.end(), hp.big_part[r].begin(), hp.big_part[r].end());
@@ -623,17 +631,24 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     // goes to one launch with a table for any degree of the tier
     if ((rc = mark_on(s, 4, 0))) return rc;
     const FailList none{nullptr, nullptr};
-    static_assert(kBigParts == 5 && kBigPartThreads[0] == 256 && kBigPartThreads[1] == 256 &&
-                      kBigPartThreads[2] == 512 && kBigPartThreads[3] == 1024 && kBigPartThreads[4] == 1024,
-                  "the launches below follow kBigPartThreads");
+    static_assert(kBigParts == 6 && 4 * kBigPartMax[0] <= 3 * kMidCap && kBigPartMax[1] == 1024 &&
+                      kBigPartThreads[2] == 256 && kBigPartThreads[3] == 512 && kBigPartThreads[4] == 1024 &&
+                      kBigPartThreads[5] == 1024,
+                  "the launches below follow kBigPartMax and kBigPartThreads");
     // unweighted counts fit 16 bits: the claim-first 16-bit tables (and
     // S::kSMThreads threads per SM) fit more blocks, and with 32-register
     // scores the 2049..4096 range runs 1024-thread blocks (measured 9 %
     // faster than 512: one batch of four entries a thread covers its rows)
     constexpr bool k16 = !W && S::kPacked;
+    // 32-bit layered scores count the first range as the mid tier does, a warp
+    // per vertex (the table at most three quarters full, far less where labels
+    // of volume 1 stay out of it): a block's barriers cost more than its rows
+    // of about 300 entries (R-MAT s22, MEASURED_384).  The other scores count
+    // it with the second range.
+    constexpr bool kWarps = S::kLV;
     for (int r = 0; r < kBigParts; ++r) {
-      const Verts& vs = p.big_part[r];
-      if (!vs.n) continue;
+      const Verts& vs = !kWarps && r == 1 && !p.merged ? p.big_first : p.big_part[r];
+      if (!vs.n || (!kWarps && r == 0 && !p.merged)) continue;
       const TierWork tw{vs, none, none, 1};
       if (p.merged && kBigPartMax[r] <= 4096 && !L.big_staged) {
         if ((rc = launch_big_merged<W>(a, TierWork{p.big_low, none, none, 1}, score, s))) return rc;
@@ -641,34 +656,40 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
         while (r + 1 < kBigParts && kBigPartMax[r + 1] <= 4096) ++r;  // the launch covered them
         continue;
       }
-      const size_t smr = 4ull * kBigPartMax[r] * sizeof(uint32_t);
+      // a table holds pow2(2 * the largest degree) slots
+      const int32_t most = r == 0 ? 512 : kBigPartMax[r];
+      static_assert(kBigPartMax[0] <= 512, "the first range's table");
+      const size_t smr = 4ull * most * sizeof(uint32_t);
       const unsigned grid = (unsigned)std::min<int64_t>(vs.n, kMaxGrid);
-      if (k16 && r < kBigParts - 1) {
-        const size_t sm16 = 12ull * kBigPartMax[r];  // 2*max slots of 4 + 2 bytes
+      if (kWarps && r == 0 && !L.big_staged) {
+        k_mid<kMidCap, kMidNT, W, S><<<(unsigned)std::min<int64_t>(cdiv(vs.n, kMidNT / 32), kMaxGrid), kMidNT, 0, s>>>(
+            a, tw, score);
+      } else if (k16 && r < kBigParts - 1) {
+        const size_t sm16 = 12ull * most;  // 2*max slots of 4 + 2 bytes
         bool staged = false;
         if constexpr (S::kPacked && !S::kKeep) {
-          if (r == 0 && L.big_staged && kBigPartMax[0] <= kStagedRow) {
+          if (r <= 1 && L.big_staged && kBigPartMax[1] <= kStagedRow) {
             // rows staged in shared memory by bulk copies, one vertex ahead
             k_big_staged<256, S><<<grid, 256, sm16, s>>>(a, tw, score);
             staged = true;
           }
         }
         if (staged) {
-        } else if (r <= 1) {
+        } else if (r <= 2) {
           k_big<256, false, S, true><<<grid, 256, sm16, s>>>(a, tw, score);
-        } else if (r == 2 && S::kSMThreads < 2048) {  // 40-register scores: 512 threads, three blocks per SM
+        } else if (r == 3 && S::kSMThreads < 2048) {  // 40-register scores: 512 threads, three blocks per SM
           if ((rc = allow_smem(k_big<512, false, S, true>, sm16))) return rc;
           k_big<512, false, S, true><<<grid, 512, sm16, s>>>(a, tw, score);
         } else {  // 2049..8192: 1024 threads cover a row in one batch (48 / 96 KB tables, two blocks per SM)
           if ((rc = allow_smem(k_big<1024, false, S, true>, sm16))) return rc;
           k_big<1024, false, S, true><<<grid, 1024, sm16, s>>>(a, tw, score);
         }
-      } else if (r < 2) {
+      } else if (r < 3) {
         k_big<256, W, S><<<grid, 256, smr, s>>>(a, tw, score);
-      } else if (r == 2) {
+      } else if (r == 3) {
         if ((rc = allow_smem(k_big<512, W, S>, smr))) return rc;
         k_big<512, W, S><<<grid, 512, smr, s>>>(a, tw, score);
-      } else if (r == 3) {
+      } else if (r == 4) {
         if ((rc = allow_smem(k_big<1024, W, S>, smr))) return rc;
         k_big<1024, W, S><<<grid, 1024, smr, s>>>(a, tw, score);
       } else if constexpr (!W) {  // the 16-bit range of unweighted graphs, load-first

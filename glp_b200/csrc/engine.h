@@ -34,10 +34,10 @@ constexpr int kMidCap = 512, kBigCap = 16384;
 // The last range counts unweighted graphs with 16-bit counts (k_big<...,
 // C16>) up to 24576; weighted graphs count it with 32-bit counts in a
 // kBigCap-slot table (128 KB) and so cap big_max at kBigMaxWeighted.
-constexpr int kBigParts = 5;
-constexpr int kBigPartMax[kBigParts] = {1024, 2048, 4096, 8192, 24576};
-constexpr int kBigLowParts = 3;  // ranges up to 4096 (merged plans)
-constexpr int kBigPartThreads[kBigParts] = {256, 256, 512, 1024, 1024};
+constexpr int kBigParts = 6;
+constexpr int kBigPartMax[kBigParts] = {384, 1024, 2048, 4096, 8192, 24576};
+constexpr int kBigLowParts = 4;  // ranges up to 4096 (merged plans)
+constexpr int kBigPartThreads[kBigParts] = {256, 256, 256, 512, 1024, 1024};
 // Graphs of at most this many non-isolated vertices run merged tiers: a step
 // of theirs is bound by its launches (see DevicePlan::merged).
 constexpr int64_t kSmallGraph = 1 << 18;
@@ -80,7 +80,7 @@ struct DevicePlan {
   TierParams tiers;
   bool valid = false;
   Verts tiny{}, g16{}, g32{}, mid{}, big{}, mb{}, pair{}, mid_rest{}, mb_rest{},
-      big_low{}, big_part[kBigParts]{};
+      big_low{}, big_first{}, big_part[kBigParts]{};
   FailList fmid{}, fbig{};
   FailList fscreen{};  // big-tier vertices a summary screen left to the exact kernel
   // list counters: [majority mid, majority big, frontier tiny, g16, g32, mid,
