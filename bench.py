@@ -320,7 +320,7 @@ def run_reference(args, ws, rank):
 # the engine's default step-mode thresholds (glp_params majority_permille /
 # frontier_permille left at 0): a step after the first counts every vertex
 # only when the previous step changed at least this many labels per 1000
-# vertices (the rule of k_step_mode)
+# vertices (the rule of k_step_begin)
 MAJORITY_PERMILLE = 500
 
 

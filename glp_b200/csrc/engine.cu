@@ -173,7 +173,8 @@ int tiers_for_graph(const glp_params* p, bool weighted, TierParams* t) {
 
 // Degree tiers; hubs get ceil(3*deg / kHubTable) hash buckets (one work item
 // each) and streaming chunks of hub_chunk edges.
-void build_host_plan(const int32_t* off, int32_t n, const TierParams& t, HostPlan* hp) {
+void build_host_plan(const int32_t* off, int32_t n, const TierParams& t, HostPlan* hp, bool merged) {
+  const int32_t tiny_max = merged ? 0 : t.tiny_max, g16_max = merged ? 0 : 16;
   *hp = HostPlan{};
   for (int32_t v = 0; v < n; ++v) {
     const int32_t d = off[v + 1] - off[v];
@@ -181,10 +182,10 @@ void build_host_plan(const int32_t* off, int32_t n, const TierParams& t, HostPla
     if (d == 0) {
       hp->isolated++;
       tier = 0;
-    } else if (d <= t.tiny_max) {
+    } else if (d <= tiny_max) {
       hp->tiny.push_back(v);
       tier = 1;
-    } else if (d <= 16) {
+    } else if (d <= g16_max) {
       hp->g16.push_back(v);
       tier = 2;
     } else if (d <= 32) {
@@ -286,6 +287,13 @@ static int device_bounds(glp_graph* g, const int32_t* thr, int k, int32_t* out);
 // Range-mode tier of a degree-sorted graph.
 static Verts range_verts(int32_t lo, int32_t hi) { return Verts{nullptr, lo, hi > lo ? hi - lo : 0}; }
 
+// Two ascending id lists in one.
+static std::vector<int32_t> merge_ids(const std::vector<int32_t>& a, const std::vector<int32_t>& b) {
+  std::vector<int32_t> out(a.size() + b.size());
+  std::merge(a.begin(), a.end(), b.begin(), b.end(), out.begin());
+  return out;
+}
+
 static int ensure_plan(glp_graph* g, const TierParams& t) {
   if (g->plan.valid && g->plan.tiers == t) return GLP_OK;
   free_plan(&g->plan);
@@ -337,16 +345,9 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     p.isolated = g->n - b[kBigParts + 4];
   } else {
     if ((rc = ensure_host_offsets(g))) return rc;
-    build_host_plan(g->h_off.data(), g->n, t, &hp);
+    p.merged = g->n <= kSmallGraph;
+    build_host_plan(g->h_off.data(), g->n, t, &hp, p.merged);
     p.isolated = hp.isolated;
-    p.merged = g->n - hp.isolated <= kSmallGraph;
-    if (p.merged) {
-      for (std::vector<int32_t>* v : {&hp.g16, &hp.tiny}) {
-        hp.g32.insert(hp.g32.end(), v->begin(), v->end());
-        v->clear();
-      }
-      std::sort(hp.g32.begin(), hp.g32.end());
-    }
     if ((rc = upload_verts(&p, hp.tiny, &p.tiny)) || (rc = upload_verts(&p, hp.g16, &p.g16)) ||
         (rc = upload_verts(&p, hp.g32, &p.g32)) || (rc = upload_verts(&p, hp.mid, &p.mid)) ||
         (rc = upload_verts(&p, hp.big, &p.big)) || (rc = upload_verts(&p, hp.mb, &p.mb)) ||
@@ -360,25 +361,20 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
         free_plan(&p);
         return rc;
       }
-    std::vector<int32_t> first = hp.big_part[0];
-    first.insert(first.end(), hp.big_part[1].begin(), hp.big_part[1].end());
-    std::sort(first.begin(), first.end());
-    if ((rc = upload_verts(&p, first, &p.big_first))) {
+    std::vector<int32_t> low = merge_ids(hp.big_part[0], hp.big_part[1]);
+    if ((rc = upload_verts(&p, low, &p.big_first))) {
       free_plan(&p);
       return rc;
     }
-    if (p.merged) {
-      std::vector<int32_t> low;
-      for (int r = 0; r < kBigLowParts; ++r) low.insert(low.end(), hp.big_part[r].begin(), hp.big_part[r].end());
-      std::sort(low.begin(), low.end());
-      if ((rc = upload_verts(&p, low, &p.big_low))) {
-        free_plan(&p);
-        return rc;
-      }
+    for (int r = 2; r < kBigLowParts; ++r) low = merge_ids(low, hp.big_part[r]);
+    if ((rc = upload_verts(&p, low, &p.big_low))) {
+      free_plan(&p);
+      return rc;
     }
   }
   n_mid = p.mid.n;
   n_big = p.big.n;
+  p.merged_big = p.big.n <= kFewBig;
   ntier[0] = p.tiny.n;
   ntier[1] = p.g16.n;
   ntier[2] = p.g32.n;
@@ -647,10 +643,10 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     // it with the second range.
     constexpr bool kWarps = S::kLV;
     for (int r = 0; r < kBigParts; ++r) {
-      const Verts& vs = !kWarps && r == 1 && !p.merged ? p.big_first : p.big_part[r];
-      if (!vs.n || (!kWarps && r == 0 && !p.merged)) continue;
+      const Verts& vs = !kWarps && r == 1 && !p.merged_big ? p.big_first : p.big_part[r];
+      if (!vs.n || (!kWarps && r == 0 && !p.merged_big)) continue;
       const TierWork tw{vs, none, none, 1};
-      if (p.merged && kBigPartMax[r] <= 4096 && !L.big_staged) {
+      if (p.merged_big && kBigPartMax[r] <= 4096 && !L.big_staged) {
         if ((rc = launch_big_merged<W>(a, TierWork{p.big_low, none, none, 1}, score, s))) return rc;
         ++*launches;
         while (r + 1 < kBigParts && kBigPartMax[r + 1] <= 4096) ++r;  // the launch covered them

@@ -30,7 +30,9 @@ constexpr int kMidCap = 512, kBigCap = 16384;
 // In full mode the big tier runs as one launch per degree range: range r
 // holds degrees up to kBigPartMax[r] (and above the previous range), counted
 // by kBigPartThreads[r]-thread blocks whose tables hold 2*kBigPartMax[r]
-// slots, so that a range's table fits as many blocks per SM as it can.
+// slots, so that a range's table fits as many blocks per SM as it can (32-bit
+// layered scores: the first range by warps, launch_step; the others count the
+// first two together).
 // The last range counts unweighted graphs with 16-bit counts (k_big<...,
 // C16>) up to 24576; weighted graphs count it with 32-bit counts in a
 // kBigCap-slot table (128 KB) and so cap big_max at kBigMaxWeighted.
@@ -38,9 +40,14 @@ constexpr int kBigParts = 6;
 constexpr int kBigPartMax[kBigParts] = {384, 1024, 2048, 4096, 8192, 24576};
 constexpr int kBigLowParts = 4;  // ranges up to 4096 (merged plans)
 constexpr int kBigPartThreads[kBigParts] = {256, 256, 256, 512, 1024, 1024};
-// Graphs of at most this many non-isolated vertices run merged tiers: a step
-// of theirs is bound by its launches (see DevicePlan::merged).
-constexpr int64_t kSmallGraph = 1 << 18;
+// A step of a small graph is bound by its launches.  Up to kSmallGraph
+// non-isolated vertices (vertices, where they are not degree-sorted) the small
+// tiers run as one (planted graphs, 20 steps: 200 k vertices 975 -> 740 us,
+// 800 k 1426 -> 1155), and up to kFewBig big vertices so do the big tier's
+// ranges to 4096 (R-MAT s15, 576 of them, 657 -> 555 us with both; s18, 4048,
+// would take 1000 -> 1035: its blocks fill the GPU).
+constexpr int64_t kSmallGraph = 1 << 20;
+constexpr int32_t kFewBig = 2048;
 constexpr int kBigMaxWeighted = 12288, kBigMaxUnweighted = 24576;
 static_assert(kBigCap == (int)kBig32Slots, "the engine sizes 32-bit big tables as k_big caps them");
 
@@ -73,7 +80,8 @@ struct HostPlan {
   std::vector<int32_t> item_hub, item_bucket;
   int64_t hub_labels = 0;
 };
-void build_host_plan(const int32_t* off, int32_t n, const TierParams& t, HostPlan* hp);
+// merged: every degree up to 32 goes to g32.
+void build_host_plan(const int32_t* off, int32_t n, const TierParams& t, HostPlan* hp, bool merged = false);
 
 struct DevicePlan {
   cudaStream_t setup = nullptr;  // stream of the set-up copies (the handle's)
@@ -98,9 +106,8 @@ struct DevicePlan {
   bool mid_c16 = true;  // mid counts fit 16 bits (unweighted, or small weight sums)
   int32_t n_hubs = 0, n_chunks = 0;
   int64_t isolated = 0;
-  // few vertices (kSmallGraph): the small tiers are one (g32) and the big tier's
-  // ranges up to 4096 one launch, since launches bound such a graph's steps
-  bool merged = false;
+  bool merged = false;      // few vertices (kSmallGraph): the small tiers are one, g32
+  bool merged_big = false;  // few big vertices (kFewBig): the ranges up to 4096 are one launch, big_low
   bool sorted = false;  // degrees never increase along the ids: every tier is a range, isolated vertices last
   HubPlan hub{};
   BigBound bb{};  // count bounds of a contiguous big tier (n = 0: the tier is an id list)

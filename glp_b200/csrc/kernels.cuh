@@ -11,7 +11,10 @@
 // Tiers (chosen by the host planner from the degree):
 //   small (1..32)      : one thread per vertex, labels sorted in registers;
 //                        three launches (<= 8, <= 16, <= 32)
+//                        (one up to 2^20 vertices); two threads per vertex for
+//                        33..64 of unweighted classic-type scores
 //   mid   (33..256)    : one warp per vertex, per-warp shared-memory table
+//                        (32-bit layered scores: to 384)
 //   big   (257..24576) : one block per vertex, block shared-memory table
 //   hub   (above big)  : labels gathered once and sorted into hash buckets,
 //                        one block per (hub, bucket) with a shared table
