@@ -1447,7 +1447,9 @@ __global__ void k_hub_offsets(HubPlan hp) {
 
 // Places the gathered labels bucket-contiguously: a block counts its labels
 // per bucket, reserves each bucket's range with one global add, then every
-// label takes a slot of its bucket's range.
+// label takes a slot of its bucket's range.  Four entries a thread and round,
+// their loads in flight together (one at a time, a branch on each label: 32 us
+// a step instead of 20 on weighted R-MAT s20).
 template <int NT, bool W>
 __global__ void __launch_bounds__(NT) k_hub_scatter(StepArgs a, HubPlan hp, int32_t nchunks) {
   extern __shared__ uint32_t sh[];  // [max_nb] counts, then [max_nb] cursors
@@ -1457,26 +1459,40 @@ __global__ void __launch_bounds__(NT) k_hub_scatter(StepArgs a, HubPlan hp, int3
     const int32_t h = hp.chunk_hub[c];
     if (hp.hub_state[h]) continue;  // block-uniform
     const uint32_t nb = (uint32_t)hp.hub_nb[h];
-    const int32_t cb = hp.chunk_begin[c], ce = hp.chunk_end[c];
+    const int32_t cb = hp.chunk_begin[c], len = hp.chunk_end[c] - cb;
     const int64_t lb = hp.hub_lbase[h];
     const int64_t base = lb - a.off[hp.hub_v[h]];
+    const int32_t* lab = hp.hlab + base + cb;
     const int32_t item0 = hp.hub_item0[h];
     for (uint32_t b = threadIdx.x; b < nb; b += NT) cnt[b] = 0;
     __syncthreads();
-    for (int32_t j = cb + threadIdx.x; j < ce; j += NT) {
-      const int32_t l = hp.hlab[base + j];
-      if (l >= 0) atomicAdd(cnt + (nb > 1 ? hub_bucket_of((uint32_t)l + 1u, nb) : 0u), 1u);
+    for (int32_t i0 = threadIdx.x; i0 < len; i0 += 4 * NT) {
+      int32_t l[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) l[q] = i0 + q * NT < len ? lab[i0 + q * NT] : -1;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (l[q] >= 0) atomicAdd(cnt + (nb > 1 ? hub_bucket_of((uint32_t)l[q] + 1u, nb) : 0u), 1u);
     }
     __syncthreads();
     for (uint32_t b = threadIdx.x; b < nb; b += NT) cur[b] = cnt[b] ? atomicAdd(hp.bcur + item0 + b, cnt[b]) : 0u;
     __syncthreads();
-    for (int32_t j = cb + threadIdx.x; j < ce; j += NT) {
-      const int32_t l = hp.hlab[base + j];
-      if (l < 0) continue;
-      const uint32_t b = nb > 1 ? hub_bucket_of((uint32_t)l + 1u, nb) : 0u;
-      const uint32_t pos = atomicAdd(cur + b, 1u);
-      hp.hsort[lb + pos] = l;
-      if (W) hp.hsw[lb + pos] = hp.hw[base + j];
+    for (int32_t i0 = threadIdx.x; i0 < len; i0 += 4 * NT) {
+      int32_t l[4], w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const bool in = i0 + q * NT < len;
+        l[q] = in ? lab[i0 + q * NT] : -1;
+        w[q] = W && in ? hp.hw[base + cb + i0 + q * NT] : 0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (l[q] < 0) continue;
+        const uint32_t b = nb > 1 ? hub_bucket_of((uint32_t)l[q] + 1u, nb) : 0u;
+        const uint32_t pos = atomicAdd(cur + b, 1u);
+        hp.hsort[lb + pos] = l[q];
+        if (W) hp.hsw[lb + pos] = w[q];
+      }
     }
     __syncthreads();
   }
