@@ -965,14 +965,16 @@ static int ensure_sorted(glp_graph* g) {
   return GLP_OK;
 }
 
-// Exact first step when the labels are the vertex ids and rows are strictly
-// ascending: unweighted, the row's last column (k_first_step); weighted, the
-// row's largest (weight, label), per tier (launch_first_keyed).
-// Per tier, the neighbour of largest key: a thread per vertex up to degree 8
-// (eight loads in flight), eight lanes per vertex up to 32 (whole sectors; the
-// planted 2M layer start, weighted, 0.27 -> 0.155 ms; at degree 8 and below
-// they idle: R-MAT s22 0.08 -> 0.13), a warp per mid and big vertex, a block
-// per hub.
+// The first step when the labels are the vertex ids and rows are strictly
+// ascending, where the neighbour of largest key wins (weighted classic and
+// layered scores; unweighted, it is the row's last column: k_first_step).  Per
+// tier: a thread per vertex up to degree 8 (eight loads in flight), eight lanes
+// per vertex up to 32 (whole sectors; the planted 2M layer start, weighted, 0.27
+// -> 0.155 ms; at degree 8 and below they idle: R-MAT s22 0.08 -> 0.13), a warp
+// per vertex up to 1024, a block above and for the hubs.  Up to kSmallGraph
+// vertices a block per big vertex: the step waits for the longest rows, and a
+// launch a range costs more than the warps save (mid and big tier of the five
+// first steps of weighted layered R-MAT s20: 1.4 ms by warps alone, 0.6 so).
 template <class K>
 static int launch_first_keyed(const DevicePlan& p, const StepArgs& a, const K& key, cudaStream_t s,
                               int64_t* launches) {
@@ -987,12 +989,21 @@ static int launch_first_keyed(const DevicePlan& p, const StepArgs& a, const K& k
                                                                                                             key);
       ++*launches;
     }
-  for (const Verts* vs : {&p.mid, &p.big})
+  const Verts none{};
+  for (const Verts* vs : {&p.mid, p.merged ? &none : &p.big_first})
     if (vs->n) {
       k_first_step_w<32, K><<<(unsigned)std::min<int64_t>(cdiv((int64_t)vs->n * 32, 256), kMaxGrid), 256, 0, s>>>(a, *vs,
                                                                                                               key);
       ++*launches;
     }
+  auto by_blocks = [&](const Verts& vs) {
+    if (!vs.n) return;
+    k_first_step_w_block<256, K><<<(unsigned)std::min<int64_t>(vs.n, kMaxGrid), 256, 0, s>>>(a, vs, key);
+    ++*launches;
+  };
+  if (p.merged) by_blocks(p.big);
+  else
+    for (int r = 2; r < kBigParts; ++r) by_blocks(p.big_part[r]);
   if (p.n_hubs) {
     k_first_step_w_block<1024, K><<<(unsigned)p.n_hubs, 1024, 0, s>>>(a, Verts{p.hub.hub_v, 0, p.n_hubs}, key);
     ++*launches;
