@@ -676,7 +676,7 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
         } else if (r == 3 && S::kSMThreads < 2048) {  // 40-register scores: 512 threads, three blocks per SM
           if ((rc = allow_smem(k_big<512, false, S, true>, sm16))) return rc;
           k_big<512, false, S, true><<<grid, 512, sm16, s>>>(a, tw, score);
-        } else {  // 2049..8192: 1024 threads cover a row in one batch (48 / 96 KB tables, two blocks per SM)
+        } else {  // 2049..8192: 1024 threads cover a row in one batch (48 / 96 KB tables)
           if ((rc = allow_smem(k_big<1024, false, S, true>, sm16))) return rc;
           k_big<1024, false, S, true><<<grid, 1024, sm16, s>>>(a, tw, score);
         }

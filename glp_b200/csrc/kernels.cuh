@@ -576,15 +576,16 @@ __device__ __forceinline__ void count_chunk(bool has, int32_t lab, uint32_t wt, 
 // 85 % of the entries of a layered step have such labels (most vertices change
 // to a label of their own neighbourhood every step), and a chunk of the table
 // costs the same however few of its lanes have an entry.
+template <bool W>
 struct ChunkRing {
   int2 lv[64];
-  uint32_t w[64];
+  uint32_t w[W ? 64 : 1];
 };
 template <bool W>
 struct ChunkQueue {
-  ChunkRing* ring;
+  ChunkRing<W>* ring;
   uint32_t head = 0, fill = 0;  // warp-uniform
-  __device__ __forceinline__ explicit ChunkQueue(ChunkRing* r) : ring(r) {}
+  __device__ __forceinline__ explicit ChunkQueue(ChunkRing<W>* r) : ring(r) {}
   // Counts the first `n` waiting entries; every lane takes part.
   template <class S, class Ins, class B>
   __device__ __forceinline__ void count(uint32_t n, const S& score, const Ins& insert, B& best, bool& fail, bool scan,
@@ -749,7 +750,7 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
   __shared__ __align__(16) uint32_t skeys[NW][CAP];
   __shared__ __align__(16) uint32_t svals[NW][C16 ? CAP / 2 : CAP];
   __shared__ int32_t cbuf[NW][32];  // changed vertices not yet listed
-  __shared__ ChunkRing rings[S::kLV ? NW : 1];
+  __shared__ ChunkRing<W> rings[S::kLV ? NW : 1];
   uint32_t ncb = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int32_t mode = step_mode(a);
@@ -909,12 +910,12 @@ constexpr int32_t kMergeDegree = 8192;
 // CF (with C16): claim-first inserts (table_claim_insert).  Off, a C16
 // table counts load-first; the top degree range runs so, its tables up to
 // three quarters full, where a CAS per probe measured slower.
-// 1024-thread blocks of packed scores run two to an SM at 32 registers; the
-// 32-bit layered score spills there (36-52 bytes) and still measured faster
-// than one block at 64 (layered R-MAT s24 big tier 2.88 -> 2.70 ms per
-// iteration)
+// 1024-thread blocks of packed scores run two to an SM at 32 registers; those
+// of the 32-bit layered score one at 64, where they do not spill: their rings
+// and a 96 KB table leave no room worth having for a second (layered R-MAT
+// s24, five layers of ten steps: 193.7 -> 187.0 ms, s22 45.9 -> 45.2).
 template <int NT, bool W, class S, bool C16 = false, bool CF = C16>
-__global__ void __launch_bounds__(NT, (!W ? ((NT == 1024 && S::kPacked) ? 2048 : S::kSMThreads)
+__global__ void __launch_bounds__(NT, (!W ? (NT == 1024 && S::kPacked ? (S::kLV ? 1024 : 2048) : S::kSMThreads)
                                           : (S::kSMThreads == 2048 && NT <= 512) ? 1536 : 1024) / NT)
     k_big(StepArgs a, TierWork tw, S score) {
   static_assert(!(C16 && W), "16-bit counts hold unweighted counts only");
@@ -922,7 +923,7 @@ __global__ void __launch_bounds__(NT, (!W ? ((NT == 1024 && S::kPacked) ? 2048 :
   const bool scan = S::kScan && scan_scores(a);
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ int32_t cbuf[64];  // changed vertices not yet listed (thread 0's)
-  __shared__ ChunkRing rings[S::kLV ? NT / 32 : 1];
+  __shared__ ChunkRing<W> rings[S::kLV ? NT / 32 : 1];
   uint32_t ncb = 0;
   __shared__ Best red[32];
   // packed scores: one slot per vertex parity, so thread 0 can read vertex
