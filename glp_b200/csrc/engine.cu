@@ -599,6 +599,22 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     if ((rc = mark_on(s, 7, 1))) return rc;
     ++*launches;
   }
+  // Weighted layered scores up to kRingGraph vertices count the mid tier
+  // without rings and the first big range by blocks: the rings' shared memory
+  // leaves the kernels beside them little L1, and there are too few rows to
+  // make up for it (five layers of ten steps, with both and without: R-MAT s20
+  // 22.7 and 20.9 ms, s21 37.8 and 36.1, s22 74.2 and 81.2).
+  const bool ring = !W || a.n - p.isolated > kRingGraph;
+  auto count_mid = [&](auto c16, const TierWork& tw, unsigned grid) {
+    constexpr bool k16c = decltype(c16)::value;
+    if constexpr (W && S::kLV) {
+      if (!ring) {
+        k_mid<kMidCap, kMidNT, W, S, k16c, false, false><<<grid, kMidNT, 0, s>>>(a, tw, score);
+        return;
+      }
+    }
+    k_mid<kMidCap, kMidNT, W, S, k16c><<<grid, kMidNT, 0, s>>>(a, tw, score);
+  };
   bool screened = false;
   if constexpr (!S::kKeep) screened = p.big.n && L.backend != GLP_BACKEND_EXACT;
   if (screened) {
@@ -639,12 +655,12 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     // 32-bit layered scores count the first range as the mid tier does, a warp
     // per vertex (the table at most three quarters full, far less where labels
     // of volume 1 stay out of it): a block's barriers cost more than its rows
-    // of about 300 entries (R-MAT s22, MEASURED_384).  The other scores count
-    // it with the second range.
-    constexpr bool kWarps = S::kLV;
+    // of about 300 entries (R-MAT s22, five layers of ten steps: 53.2 ms by
+    // blocks, 46.0 by warps).  The other scores count it with the second range.
+    const bool warps = S::kLV && ring;
     for (int r = 0; r < kBigParts; ++r) {
-      const Verts& vs = !kWarps && r == 1 && !p.merged_big ? p.big_first : p.big_part[r];
-      if (!vs.n || (!kWarps && r == 0 && !p.merged_big)) continue;
+      const Verts& vs = !warps && r == 1 && !p.merged_big ? p.big_first : p.big_part[r];
+      if (!vs.n || (!warps && r == 0 && !p.merged_big)) continue;
       const TierWork tw{vs, none, none, 1};
       if (p.merged_big && kBigPartMax[r] <= 4096 && !L.big_staged) {
         if ((rc = launch_big_merged<W>(a, TierWork{p.big_low, none, none, 1}, score, s))) return rc;
@@ -657,9 +673,8 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
       static_assert(kBigPartMax[0] <= 512, "the first range's table");
       const size_t smr = 4ull * most * sizeof(uint32_t);
       const unsigned grid = (unsigned)std::min<int64_t>(vs.n, kMaxGrid);
-      if (kWarps && r == 0 && !L.big_staged) {
-        k_mid<kMidCap, kMidNT, W, S><<<(unsigned)std::min<int64_t>(cdiv(vs.n, kMidNT / 32), kMaxGrid), kMidNT, 0, s>>>(
-            a, tw, score);
+      if (warps && r == 0 && !L.big_staged) {
+        count_mid(std::bool_constant<S::kPacked && !W>{}, tw, (unsigned)std::min<int64_t>(cdiv(vs.n, kMidNT / 32), kMaxGrid));
       } else if (k16 && r < kBigParts - 1) {
         const size_t sm16 = 12ull * most;  // 2*max slots of 4 + 2 bytes
         bool staged = false;
@@ -726,7 +741,7 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     }
     if constexpr (W && S::kPacked) {
       c16w = p.mid_c16;
-      if (c16w) k_mid<kMidCap, kMidNT, W, S, true><<<grid, kMidNT, 0, s>>>(a, mw, score);
+      if (c16w) count_mid(std::true_type{}, mw, grid);
     }
     if (!c16w) {
       // the next vertex's first batch in flight while counting: unweighted
@@ -735,7 +750,7 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
         if (L.mid_prefetch) k_mid<kMidCap, kMidNT, W, S, true, true><<<grid, kMidNT, 0, s>>>(a, mw, score);
         else k_mid<kMidCap, kMidNT, W, S><<<grid, kMidNT, 0, s>>>(a, mw, score);
       } else {
-        k_mid<kMidCap, kMidNT, W, S><<<grid, kMidNT, 0, s>>>(a, mw, score);
+        count_mid(std::bool_constant<S::kPacked && !W>{}, mw, grid);
       }
     }
     if ((rc = mark_on(s, 3, 1))) return rc;

@@ -31,7 +31,7 @@ constexpr int kMidCap = 512, kBigCap = 16384;
 // holds degrees up to kBigPartMax[r] (and above the previous range), counted
 // by kBigPartThreads[r]-thread blocks whose tables hold 2*kBigPartMax[r]
 // slots, so that a range's table fits as many blocks per SM as it can (32-bit
-// layered scores: the first range by warps, launch_step; the others count the
+// layered scores: the first range by warps where launch_step says; the others count the
 // first two together).
 // The last range counts unweighted graphs with 16-bit counts (k_big<...,
 // C16>) up to 24576; weighted graphs count it with 32-bit counts in a
@@ -48,6 +48,9 @@ constexpr int kBigPartThreads[kBigParts] = {256, 256, 256, 512, 1024, 1024};
 // would take 1000 -> 1035: its blocks fill the GPU).
 constexpr int64_t kSmallGraph = 1 << 20;
 constexpr int32_t kFewBig = 2048;
+// Weighted layered scores: rings and the first big range by warps above this
+// many non-isolated vertices (launch_step).
+constexpr int64_t kRingGraph = 1 << 21;
 constexpr int kBigMaxWeighted = 12288, kBigMaxUnweighted = 24576;
 static_assert(kBigCap == (int)kBig32Slots, "the engine sizes 32-bit big tables as k_big caps them");
 

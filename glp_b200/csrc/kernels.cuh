@@ -733,11 +733,12 @@ __global__ void __launch_bounds__(256) k_major_warp(StepArgs a, Verts vs, int32_
 // C16: 16-bit counts (unweighted: a count never exceeds the degree;
 // weighted: the caller knows every mid vertex's weights sum below 2^16), so
 // that the tables and 32 registers a thread fit eight blocks per SM.
+// RING: labels of volume 1 stay out of the table (ChunkQueue).
 // PF: the first batch of the warp's next vertex (its columns, then its
 // neighbour labels) is loaded before the current vertex is counted, so the
 // label gathers are in flight while the table work runs; it costs registers
 // (at most 40 a thread: six blocks per SM).
-template <int CAP, int NT, bool W, class S, bool C16 = (S::kPacked && !W), bool PF = false>
+template <int CAP, int NT, bool W, class S, bool C16 = (S::kPacked && !W), bool PF = false, bool RING = S::kLV>
 __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
                                          : (C16 ? S::kSMThreads : S::kSMThreads == 2048 ? 1536 : 1024) / NT)
     k_mid(StepArgs a, TierWork tw, S score) {
@@ -750,7 +751,7 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
   __shared__ __align__(16) uint32_t skeys[NW][CAP];
   __shared__ __align__(16) uint32_t svals[NW][C16 ? CAP / 2 : CAP];
   __shared__ int32_t cbuf[NW][32];  // changed vertices not yet listed
-  __shared__ ChunkRing<W> rings[S::kLV ? NW : 1];
+  __shared__ ChunkRing<W> rings[RING ? NW : 1];
   uint32_t ncb = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int32_t mode = step_mode(a);
@@ -828,7 +829,7 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
       return CF ? table_claim_insert<C16>(kk, vv, cap - 1, key, k, cap)
                 : table_insert_bounded<C16>(kk, vv, cap - 1, key, k, cap, nullptr, nullptr);
     };
-    ChunkQueue<W> queue(&rings[S::kLV ? warp : 0]);
+    ChunkQueue<W> queue(&rings[RING ? warp : 0]);
     for (int32_t j0 = b; j0 < e; j0 += 128) {
       int32_t lab[4], vl[4];
       uint32_t wt[4];
@@ -842,7 +843,7 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
       } else {
         load_batch(j0, e, lab, wt, vl);
       }
-      if constexpr (S::kLV) {
+      if constexpr (RING) {
         if (score.single) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
@@ -855,7 +856,7 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
         if (j0 + 32 * q < e)
           count_chunk<W, S::kLV>(lab[q] >= 0, lab[q], wt[q], score, ins, best, fail, scan, vl[q], merge);
     }
-    if constexpr (S::kLV) queue.finish(score, ins, best, fail, scan, merge);
+    if constexpr (RING) queue.finish(score, ins, best, fail, scan, merge);
     if (fail) atomicOr(a.err, kErrProbe);
     if (scan) {
       __syncwarp();
