@@ -61,6 +61,18 @@ int device_sms() {
   return sms;
 }
 
+// Bytes of the current device's L2, queried once per device (0 when the query
+// fails).
+static int64_t device_l2() {
+  static std::atomic<int> cache[64];
+  int dev = 0, bytes = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (dev >= 0 && dev < 64 && (bytes = cache[dev].load(std::memory_order_relaxed)) > 0) return bytes;
+  if (cudaDeviceGetAttribute(&bytes, cudaDevAttrL2CacheSize, dev) != cudaSuccess) return 0;
+  if (dev >= 0 && dev < 64) cache[dev].store(bytes, std::memory_order_relaxed);
+  return bytes;
+}
+
 // Device memory of graph handles comes from the device's stream-ordered pool,
 // set once per device to keep freed memory in this process (release
 // threshold at its maximum): handles created and destroyed in a loop reuse
@@ -559,7 +571,13 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
   // fork: hubs on aux[0], the small tiers on aux[1], the rest here
   GLP_CUDA(cudaEventRecord(L.fork, s));
   if (p.n_hubs) GLP_CUDA(cudaStreamWaitEvent(L.aux[0], L.fork, 0));
-  GLP_CUDA(cudaStreamWaitEvent(L.aux[1], L.fork, 0));
+  // Weighted layered scores whose (label, volume) pairs exceed the L2: the
+  // small tiers start after the big tier, which they slow by more than the
+  // overlap gains (R-MAT s24, 134 MB of pairs, five layers of ten steps: 331 ->
+  // 313 ms; unweighted s24 191.9 either way; s22, 34 MB, weighted 74.2 -> 75.5,
+  // unweighted 46.0 -> 49.3).
+  const bool late = W && S::kLV && (int64_t)a.n * (int64_t)sizeof(int2) > device_l2();
+  if (!late) GLP_CUDA(cudaStreamWaitEvent(L.aux[1], L.fork, 0));
   constexpr int kMidNT = 256, kBigNT = 256, kHubNT = 512, kBucketNT = 512;
   if (p.n_hubs) {
     const size_t sm = 2ull * kHubTable * sizeof(uint32_t);
@@ -720,6 +738,10 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
         return rc;
     }
     if ((rc = mark_on(s, 4, 1))) return rc;
+  }
+  if (late) {
+    GLP_CUDA(cudaEventRecord(L.fork, s));
+    GLP_CUDA(cudaStreamWaitEvent(L.aux[1], L.fork, 0));
   }
   if (p.mid.n) {
     if ((rc = mark_on(s, 3, 0))) return rc;

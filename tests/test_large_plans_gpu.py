@@ -6,6 +6,7 @@ import functools
 
 import numpy as np
 import pytest
+import torch
 
 from glp_b200 import _lib
 from glp_b200.engine import Graph, make_params
@@ -87,3 +88,15 @@ def test_layered_per_iteration(order, pairs, weighted):
     got = _trace(off, cols, w, _lib.METHOD_LAYERED, 3, dstar=[2, 9])
     _, _, want = O.layered_run(off, cols, [2, 9], 3, w=w, trace=True)
     np.testing.assert_array_equal(got, want)
+
+
+def test_weighted_layered_pairs_beyond_the_whole_cache():
+    """(label, volume) pairs past the L2: the small tiers follow the big tier."""
+    l2 = torch.cuda.get_device_properties(0).L2_cache_size
+    off, cols = _graph("sorted", isolated=l2 // 8 + 1000)
+    w = _weights(cols)
+    with Graph(from_numpy(off, cols, w)) as g:
+        got = g.run(_lib.METHOD_LAYERED, 3, make_params(dstar=[3]))
+    want, vol = O.layered_run(off, cols, [3], 3, w=w)[:2]
+    np.testing.assert_array_equal(got.labels, want)
+    np.testing.assert_array_equal(got.vol, vol)
