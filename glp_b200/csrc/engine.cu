@@ -511,6 +511,21 @@ template <int R, bool W, class S>
 static int launch_small(const StepArgs& a, const TierWork& tw, const S& score, cudaStream_t s) {
   const unsigned grid = (unsigned)std::min<int64_t>(cdiv(tw.all.n, kSmallNT), device_sms() * 32);
   const size_t sm = (size_t)(kSmallNT / 32) * small_words<R, W, S>() * sizeof(uint32_t);
+  if constexpr (R == 32 && !W && S::kLV) {
+    // Random reads of pairs beyond a quarter of the L2 miss it: such graphs
+    // gather labels alone and look a volume up per distinct label of a row, in
+    // an L1 of which the kernel asks half to stay a cache (planted graphs,
+    // five layers of ten steps: 10 M vertices 69.9 -> 53.5 ms, 4 M 23.2 ->
+    // 21.3, 2 M 14.1 -> 14.25; the labels alone with the default carve-out,
+    // which leaves 28 KB of L1, take 69.9 at 10 M).
+    if ((int64_t)a.n * (int64_t)sizeof(int2) > device_l2() / 4) {
+      using G = ScoreLayered32L;
+      GLP_CUDA(prefer_smem_share((const void*)k_small<R, W, G, int32_t>, 50));
+      k_small<R, W, G, int32_t><<<grid, kSmallNT, (size_t)(kSmallNT / 32) * small_words<R, W, G>() * sizeof(uint32_t),
+                                  s>>>(a, tw, G{score.vol, score.dstar});
+      return GLP_OK;
+    }
+  }
   if constexpr (W || S::kLV) {
     if (a.n < (1 << 27)) {
       GLP_CUDA(raise_smem_limit((const void*)k_small<R, W, S, uint32_t>, sm));

@@ -318,6 +318,25 @@ struct ScoreLayered32 {
   }
 };
 
+// ScoreLayered32 that gathers the labels alone and looks the volumes up, once
+// per distinct label of a row (small tiers; launch_small).
+struct ScoreLayered32L {
+  static constexpr bool kKeep = false;
+  __device__ __forceinline__ bool fixed(int32_t) const { return false; }
+  static constexpr bool kPacked = true;
+  static constexpr bool kScan = true;
+  static constexpr bool kLV = false;
+  const int32_t* vol;
+  int32_t dstar;
+  __device__ __forceinline__ void load(const StepArgs& a, int32_t c, int32_t& lab, int32_t&) const {
+    lab = ld_label(a.lin + c);
+  }
+  __device__ __forceinline__ int32_t vol_of(int32_t l) const { return __ldg(vol + l); }
+  __device__ __forceinline__ uint32_t key32(uint32_t k, int32_t v) const {
+    return (uint32_t)(dstar * (int32_t)k - v) ^ 0x80000000u;
+  }
+};
+
 // Seeded LP (method 5; seeded.cuh): classic counts over the labelled
 // neighbours only (a label of -1 is no entry), seeds fixed, and a vertex
 // without a labelled neighbour keeps its label.  The packed key is count + 1,

@@ -1,4 +1,4 @@
-// smem_attr.h -- the per-process dynamic shared memory limit of a kernel.
+// smem_attr.h -- the per-process shared memory attributes of a kernel.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -23,6 +23,22 @@ inline cudaError_t raise_smem_limit(const void* kernel, size_t bytes) {
   if (bytes <= cur) return cudaSuccess;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e == cudaSuccess) cur = bytes;
+  return e;
+}
+
+// Hints that an SM running `kernel` gives `percent` of its shared memory and
+// L1 to shared memory (once per device; the same percent in every call).
+inline cudaError_t prefer_smem_share(const void* kernel, int percent) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, int> shares;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  int& cur = shares[{dev, kernel}];
+  if (cur == percent) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+  if (e == cudaSuccess) cur = percent;
   return e;
 }
 

@@ -90,6 +90,17 @@ def test_layered_per_iteration(order, pairs, weighted):
     np.testing.assert_array_equal(got, want)
 
 
+@pytest.mark.parametrize("pairs", [0, UNMERGED])
+def test_layered_pairs_beyond_the_cache(pairs):
+    """(label, volume) pairs past a quarter of the L2: degrees 17..32 gather the
+    labels alone."""
+    l2 = torch.cuda.get_device_properties(0).L2_cache_size
+    off, cols = _graph("sorted", pairs, isolated=l2 // 32 + 1000)
+    got = _trace(off, cols, None, _lib.METHOD_LAYERED, 2, dstar=[2, 17])
+    _, _, want = O.layered_run(off, cols, [2, 17], 2, trace=True)
+    np.testing.assert_array_equal(got, want)
+
+
 def test_weighted_layered_pairs_beyond_the_whole_cache():
     """(label, volume) pairs past the L2: the small tiers follow the big tier."""
     l2 = torch.cuda.get_device_properties(0).L2_cache_size
