@@ -404,15 +404,65 @@ __global__ void k_starts(const uint64_t* __restrict__ keys, int64_t m, int64_t r
   }
 }
 
+// Claims or finds key's slot in a table of kDedupeSlots; false past kProbeMost
+// probes.  *fresh grows when this call claimed it.
+constexpr int kDedupeSlots = 2048, kDedupeMean = 1024, kProbeMost = 128;
+__device__ __forceinline__ bool dedupe_insert(uint64_t* table, uint64_t key, uint64_t hash, uint32_t* fresh) {
+  uint32_t slot = (uint32_t)hash & (kDedupeSlots - 1);
+  for (int probe = 0; probe < kProbeMost; ++probe) {
+    const uint64_t prev = atomicCAS((unsigned long long*)&table[slot], (unsigned long long)kNoKey,
+                                    (unsigned long long)key);
+    if (prev == kNoKey) ++*fresh;
+    if (prev == kNoKey || prev == key) return true;
+    slot = (slot + 1) & (kDedupeSlots - 1);
+  }
+  return false;
+}
+
+// A pair that repeats fills its bucket with copies, and a bucket has one block.
+// So the tiles of kSortTile keys that lie within one bucket (an ordinary bucket
+// holds none) drop their copies first, a block per tile: the distinct keys move
+// to the tile's front and left[t] is their number; a tile of too many keeps all.
+// A key already in its slot is read there, not claimed: equal claims of a warp
+// serialise.  (67 M edges, a quarter of them one pair: 53.3 -> 10.4 ms to the
+// handle; all one pair 177 -> 5.8.)
+__global__ void __launch_bounds__(kNT) k_thin(uint64_t* __restrict__ keys, HashBucket bucket,
+                                              uint32_t* __restrict__ left) {
+  __shared__ uint64_t table[kDedupeSlots];
+  __shared__ uint32_t cursor;
+  uint64_t* tile = keys + (int64_t)blockIdx.x * kSortTile;
+  if (bucket(tile[0]) != bucket(tile[kSortTile - 1])) return;  // block-uniform
+  for (int s = threadIdx.x; s < kDedupeSlots; s += kNT) table[s] = kNoKey;
+  if (threadIdx.x == 0) cursor = 0u;
+  __syncthreads();
+  uint32_t fresh = 0;
+  bool full = false;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < kSortTile; i += kNT) {
+    const uint64_t key = tile[i], h = glp::mix64(key);
+    if (*(volatile uint64_t*)&table[(uint32_t)h & (kDedupeSlots - 1)] != key)
+      full = !dedupe_insert(table, key, h, &fresh) || full;
+  }
+  if (__syncthreads_or(full)) {  // block-uniform; every key has been read
+    if (threadIdx.x == 0) left[blockIdx.x] = kSortTile;
+    return;
+  }
+  for (int s = threadIdx.x; s < kDedupeSlots; s += kNT)
+    if (table[s] != kNoKey) tile[atomicAdd(&cursor, 1u)] = table[s];
+  __syncthreads();
+  if (threadIdx.x == 0) left[blockIdx.x] = cursor;
+}
+
 // Drops duplicate keys.  A block per hash bucket (about 1000 keys) inserts
 // them in a shared table and writes the distinct ones, in no order, to `out`,
-// counting degrees.  A bucket whose keys do not fit (a probe past kProbeMost)
+// counting degrees.  Of the tiles within the bucket it takes the left[t] keys
+// that k_thin left.  A bucket whose keys do not fit (a probe past kProbeMost)
 // is split by further bits of the hash, as often as it takes: the classes
 // (level, low bits) are walked depth first, each written once.
-constexpr int kDedupeSlots = 2048, kDedupeMean = 1024, kProbeMost = 128;
 __global__ void __launch_bounds__(kNT) k_dedupe(const uint64_t* __restrict__ keys, const int32_t* __restrict__ start,
-                                                int32_t nbuckets, int idbits, int both, uint64_t* __restrict__ out,
-                                                unsigned long long* nout, int32_t* __restrict__ deg) {
+                                                const uint32_t* __restrict__ left, int32_t nbuckets, int idbits,
+                                                int both, uint64_t* __restrict__ out, unsigned long long* nout,
+                                                int32_t* __restrict__ deg) {
   __shared__ uint64_t table[kDedupeSlots];
   __shared__ uint32_t cursor;
   __shared__ unsigned long long sbase;
@@ -420,6 +470,7 @@ __global__ void __launch_bounds__(kNT) k_dedupe(const uint64_t* __restrict__ key
   const uint64_t idmask = (1ull << idbits) - 1ull;
   for (int32_t bk = blockIdx.x; bk < nbuckets; bk += gridDim.x) {
     const int32_t kb = start[bk], ke = start[bk + 1];
+    const int32_t t0 = (kb + kSortTile - 1) / kSortTile, t1 = ke / kSortTile;  // tiles within the bucket
     int level = 0;
     uint64_t cls = 0;  // keys whose (hash >> 11) & (2^level - 1) is cls
     for (bool more = true; more;) {
@@ -428,21 +479,15 @@ __global__ void __launch_bounds__(kNT) k_dedupe(const uint64_t* __restrict__ key
       __syncthreads();
       uint32_t fresh = 0;
       bool full = false;
-      for (int32_t i = kb + threadIdx.x; i < ke; i += kNT) {
-        const uint64_t key = keys[i];
+      auto put = [&](uint64_t key) {
         const uint64_t h = glp::mix64(key);  // bucket: high bits; slot: low bits; class: the bits above the slot's
-        if (((h >> 11) & ((1ull << level) - 1ull)) != cls) continue;
-        uint32_t slot = (uint32_t)h & (kDedupeSlots - 1);
-        int probe = 0;
-        for (; probe < kProbeMost; ++probe) {
-          const uint64_t prev = atomicCAS((unsigned long long*)&table[slot], (unsigned long long)kNoKey,
-                                          (unsigned long long)key);
-          if (prev == kNoKey) ++fresh;
-          if (prev == kNoKey || prev == key) break;
-          slot = (slot + 1) & (kDedupeSlots - 1);
-        }
-        full = full || probe == kProbeMost;
-      }
+        if (((h >> 11) & ((1ull << level) - 1ull)) == cls) full = !dedupe_insert(table, key, h, &fresh) || full;
+      };
+      for (int32_t i = kb + threadIdx.x; i < (t0 < t1 ? t0 * kSortTile : ke); i += kNT) put(keys[i]);
+      for (int32_t t = t0 + (threadIdx.x >> 5); t < t1; t += kNT / 32)
+        for (uint32_t i = lane; i < left[t]; i += 32) put(keys[(int64_t)t * kSortTile + i]);
+      if (t0 < t1)
+        for (int32_t i = t1 * kSortTile + threadIdx.x; i < ke; i += kNT) put(keys[i]);
       // the hash is a bijection: 53 levels would leave each slot one key
       if (__syncthreads_or(full)) {  // block-uniform
         ++level;
@@ -694,8 +739,9 @@ int ingest_edges(const int32_t* src, const int32_t* dst, int64_t count, int32_t 
       uint64_t *a = kb.p, *b = ka.p;
       if ((rc = radix_sort<HashDigit>(ka.p, &a, &b, nk0, 64 - bits, bits, so, s))) return rc;
       k_starts<<<blocks((int64_t)nbuckets + 1), kNT, 0, s>>>(a, nk0, nbuckets, HashBucket{64 - bits}, bstart.p);
+      if (nk0 >= kSortTile) k_thin<<<(unsigned)(nk0 / kSortTile), kNT, 0, s>>>(a, HashBucket{64 - bits}, hist.p);
       k_dedupe<<<(unsigned)std::min<int64_t>(nbuckets, (int64_t)device_sms() * 64), kNT, 0, s>>>(
-          a, bstart.p, nbuckets, idb, both ? 1 : 0, b, nk.p + 1, deg.p);
+          a, bstart.p, hist.p, nbuckets, idb, both ? 1 : 0, b, nk.p + 1, deg.p);
       ICUDA(cudaGetLastError());
       keys = b;
       tmp = a;
