@@ -169,6 +169,10 @@ constexpr uint32_t group_slots() {
   return p < 512u ? 2 * p : p;
 }
 
+// Labels and change flags are read by plain loads throughout: the steps of one
+// launch write them, and the read-only path (ld_label) asks for memory that
+// nothing writes while the kernel runs.
+
 // One vertex per group of G lanes (G | 32), at most G*L neighbours, L labels
 // per lane in registers.  v < 0: this group has no vertex (it still takes
 // part in the warp-wide shuffles).  keys: the group's table slice, kCap =
@@ -215,7 +219,7 @@ __device__ __forceinline__ bool group_vertex(const BatchArgs& a, int32_t v, cons
   }
 #pragma unroll
   for (int q = 0; q < L; ++q)
-    if (lab[q] >= 0 && !done) lab[q] = ld_label(lin + lab[q]);
+    if (lab[q] >= 0 && !done) lab[q] = lin[lab[q]];
   if (majority) {
     uint32_t c = 0;
 #pragma unroll
@@ -346,7 +350,7 @@ __device__ __forceinline__ bool block_vertex(const BatchArgs& a, int32_t v, cons
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      if (lab[q] >= 0) lab[q] = ld_label(lin + lab[q]);
+      if (lab[q] >= 0) lab[q] = lin[lab[q]];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (j0 + q * NT >= d) break;  // warp-uniform
@@ -448,7 +452,7 @@ __device__ __forceinline__ uint32_t sweep_threads(const BatchArgs& a, int64_t lo
         for (int g = 0; g < 8; ++g) {
           const int t = 4 * g + grp;
           in[g] = i < __shfl_sync(kFull, d, t) && (rows >> t & 1u);
-          if (in[g]) lab[g] = ld_label(lin + slab[small_at<R>(t, i)]);
+          if (in[g]) lab[g] = lin[slab[small_at<R>(t, i)]];
         }
 #pragma unroll
         for (int g = 0; g < 8; ++g)
