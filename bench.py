@@ -351,6 +351,11 @@ def full_count_roofline(plan: dict, runs: list, n: int, peak: float,
                 per[key] += float(st[it][t])
     if not per or full_steps == 0:
         return {}
+    if per.get("group32", 0.0) > 0 and per.get("tiny", 0.0) + per.get("group16", 0.0) <= 0:
+        # a small graph's one launch for degrees 1..32, timed as group32
+        plan = dict(plan)
+        for c in "ve":
+            plan[f"{c}_group32"] += plan[f"{c}_tiny"] + plan[f"{c}_group16"]
     key = max(per, key=per.get)
     n_t, m_t = plan[f"v_{key}"], plan[f"e_{key}"]
     bytes_launch = 8 * m_t + 12 * n_t

@@ -143,6 +143,7 @@ int resolve_tiers(const glp_params* p, TierParams* t) {
   if (p) {
     if (p->tiny_max > 0) d.tiny_max = p->tiny_max;
     if (p->tiny_max < 0) d.tiny_max = 0;
+    d.tiny_auto = p->tiny_max == 0;
     if (p->mid_max > 0) d.mid_max = p->mid_max;
     if (p->big_max > 0) {
       d.big_max = p->big_max;
@@ -348,7 +349,8 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     p.pair = range_verts(b[kBigParts + 5], b[kBigParts + 1]);
     p.mid_rest = range_verts(b[kBigParts], b[kBigParts + 5]);
     p.mb_rest = range_verts(b[0], b[kBigParts + 5]);
-    p.merged = b[kBigParts + 4] <= kSmallGraph;
+    p.small = b[kBigParts + 4] <= kSmallGraph;
+    p.merged = p.small && t.tiny_auto;
     p.g32 = range_verts(b[kBigParts + 1], b[kBigParts + (p.merged ? 4 : 2)]);
     if (!p.merged) {
       p.g16 = range_verts(b[kBigParts + 2], b[kBigParts + 3]);
@@ -357,7 +359,8 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     p.isolated = g->n - b[kBigParts + 4];
   } else {
     if ((rc = ensure_host_offsets(g))) return rc;
-    p.merged = g->n <= kSmallGraph;
+    p.small = g->n <= kSmallGraph;
+    p.merged = p.small && t.tiny_auto;
     build_host_plan(g->h_off.data(), g->n, t, &hp, p.merged);
     p.isolated = hp.isolated;
     if ((rc = upload_verts(&p, hp.tiny, &p.tiny)) || (rc = upload_verts(&p, hp.g16, &p.g16)) ||
@@ -1042,7 +1045,7 @@ static int launch_first_keyed(const DevicePlan& p, const StepArgs& a, const K& k
       ++*launches;
     }
   const Verts none{};
-  for (const Verts* vs : {&p.mid, p.merged ? &none : &p.big_first})
+  for (const Verts* vs : {&p.mid, p.small ? &none : &p.big_first})
     if (vs->n) {
       k_first_step_w<32, K><<<(unsigned)std::min<int64_t>(cdiv((int64_t)vs->n * 32, 256), kMaxGrid), 256, 0, s>>>(a, *vs,
                                                                                                               key);
@@ -1053,7 +1056,7 @@ static int launch_first_keyed(const DevicePlan& p, const StepArgs& a, const K& k
     k_first_step_w_block<256, K><<<(unsigned)std::min<int64_t>(vs.n, kMaxGrid), 256, 0, s>>>(a, vs, key);
     ++*launches;
   };
-  if (p.merged) by_blocks(p.big);
+  if (p.small) by_blocks(p.big);
   else
     for (int r = 2; r < kBigParts; ++r) by_blocks(p.big_part[r]);
   if (p.n_hubs) {

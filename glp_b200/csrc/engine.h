@@ -56,12 +56,13 @@ static_assert(kBigCap == (int)kBig32Slots, "the engine sizes 32-bit big tables a
 
 struct TierParams {
   int32_t tiny_max = 8;       // <= 8
+  bool tiny_auto = true;      // tiny_max not given: small graphs count the small tiers as one (kSmallGraph)
   int32_t mid_max = 256;      // <= kMidCap / 2
   int32_t big_max = kBigMaxWeighted;  // <= kBigMaxUnweighted (unweighted graphs), <= kBigMaxWeighted (weighted)
   bool big_auto = true;               // big_max not given: the largest the graph's counts allow
   int32_t hub_chunk = 16384;  // edges per hub streaming block
   bool operator==(const TierParams& o) const {
-    return tiny_max == o.tiny_max && mid_max == o.mid_max && big_max == o.big_max && hub_chunk == o.hub_chunk;
+    return tiny_max == o.tiny_max && tiny_auto == o.tiny_auto && mid_max == o.mid_max && big_max == o.big_max && hub_chunk == o.hub_chunk;
   }
 };
 int resolve_tiers(const glp_params* p, TierParams* t);
@@ -109,7 +110,8 @@ struct DevicePlan {
   bool mid_c16 = true;  // mid counts fit 16 bits (unweighted, or small weight sums)
   int32_t n_hubs = 0, n_chunks = 0;
   int64_t isolated = 0;
-  bool merged = false;      // few vertices (kSmallGraph): the small tiers are one, g32
+  bool small = false;       // few vertices (kSmallGraph)
+  bool merged = false;      // few vertices and tiny_max not given: the small tiers are one, g32
   bool merged_big = false;  // few big vertices (kFewBig): the ranges up to 4096 are one launch, big_low
   bool sorted = false;  // degrees never increase along the ids: every tier is a range, isolated vertices last
   HubPlan hub{};

@@ -84,7 +84,9 @@ typedef struct glp_params {
   /* method 4 */
   int32_t hooks;                  /* GLP_HOOKS_* */
   /* degree tiers (0 = engine default / autotuned) */
-  int32_t tiny_max;               /* thread per vertex up to this degree (<= 8) */
+  int32_t tiny_max;               /* the first of the three small tiers ends at this degree (<= 8; -1: there
+                                     is none).  0: 8, and a graph of at most 2^20 vertices counts degrees
+                                     1..32 in one launch, timed as group32 */
   int32_t mid_max;                /* warp per vertex up to this degree (32..256) */
   int32_t big_max;                /* block per vertex up to this degree (mid_max..24576 unweighted,
                                      mid_max..12288 weighted); above: hubs.  0 = the largest the
@@ -186,7 +188,8 @@ int glp_graph_info(const glp_graph* g, int32_t* n, int64_t* m, int32_t* max_degr
  * [isolated, tiny, group16, group32, mid, big, hub]; out[7]: hub hash
  * buckets; out[8..14]: CSR entries (edges) per tier in the same order;
  * out[15]: hub streaming chunks.  Mirrors the bin report of
- * prop/classicLprop.cuh:213-227. */
+ * prop/classicLprop.cuh:213-227.  (Launches may cover several tiers: see
+ * tiny_max.) */
 int glp_graph_plan(glp_graph* g, const glp_params* p, int64_t out[16]);
 /* The same plan computed from host offsets alone (no device needed),
  * planned as for an unweighted graph. */
