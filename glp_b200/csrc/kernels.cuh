@@ -1816,7 +1816,8 @@ __global__ void __launch_bounds__(256) k_check_sorted(const int32_t* __restrict_
 // listed its changed vertices (chg_in); marks carry this step's epoch, so
 // nothing is ever cleared.  The output buffer already holds the labels of
 // two steps back, which equal the current ones except for chg_in: those that
-// are not recomputed are copied.  No pass touches all n vertices.
+// are not recomputed are copied.  After few changes no pass touches all n
+// vertices (frontier_direct).
 struct Frontier {
   uint32_t* act;           // [n] epoch of the last step that marked the vertex
   uint32_t epoch;          // this step's mark (unique per step of the handle)
@@ -1824,16 +1825,28 @@ struct Frontier {
   const uint32_t* chg_in_n;
   int32_t tiny_max, g16_max, mid_max, big_max;
   FailList tier[5];        // frontier members of tiny, g16, g32, mid, big
+  __device__ __forceinline__ int tier_of(int32_t d) const {
+    return d <= tiny_max ? 0 : d <= g16_max ? 1 : d <= 32 ? 2 : d <= mid_max ? 3 : d <= big_max ? 4 : -1;
+  }
 };
+
+// Whether a frontier step lists its vertices as it marks them.  That takes an
+// atomic exchange and two gathers per entry of a changed row and an add to a
+// tier's counter per warp and 32 entries (planted 10M, 0.5 M changed vertices:
+// 0.74 ms, where marks by plain stores and a scan of all of them take 0.12); the
+// scan takes 1 ps a vertex whatever changed.  Below n / 2048 changes the listing
+// is the cheaper (60 steps of 200 M vertices in triangles, 3000 changes and
+// fewer in all but two: 23.6 ms by scans, 9.7 so; R-MAT s24 and planted 10M,
+// whose last steps change 600 ppm and fewer, are alike from n / 512 to n / 8192).
+constexpr int64_t kDirectShare = 2048;
+__device__ __forceinline__ bool frontier_direct(const StepArgs& a, uint32_t nc) { return nc * kDirectShare < a.n; }
 
 // Marks the neighbours of the changed vertices (and counts, for the big tier's
 // bounds, each of its members' changed neighbours): eight lanes per changed
 // vertex, a warp for rows above kPushRow.  A mark is a plain store: which
 // vertices are marked is collected afterwards, in id order, by
-// k_frontier_list.  (Listing a vertex when it is first marked took an atomic
-// exchange and two gathers per entry and an add to a tier's counter per warp
-// and entry group: the first frontier step of planted 10M, 0.5 M changed
-// vertices, 0.74 ms; push and list now take 0.12.)
+// k_frontier_list.  After few changes (frontier_direct) a warp per changed
+// vertex lists each vertex it is the first to mark.
 constexpr int32_t kPushRow = 256;
 __device__ __forceinline__ void push_entry(const StepArgs& a, const Frontier& f, int32_t j) {
   const int32_t x = ld_stream(a.cols + j);
@@ -1845,6 +1858,31 @@ __global__ void __launch_bounds__(256) k_frontier_push(StepArgs a, Frontier f) {
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const uint32_t nc = *f.chg_in_n;
+  if (frontier_direct(a, nc)) {
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nc; i += nw) {
+      const int32_t u = f.chg_in[i];
+      const int32_t b = a.off[u], d = a.off[u + 1] - b;
+      for (int64_t c0 = 0; c0 < d; c0 += 32) {  // warp-uniform
+        int tier = -1;
+        int32_t x = 0;
+        if (c0 + lane < d) {
+          x = ld_stream(a.cols + b + c0 + lane);
+          if (a.bb.has(x)) atomicAdd(a.bb.nchg + (x - a.bb.base), 1u);
+          if (atomicExch(f.act + x, f.epoch) != f.epoch) tier = f.tier_of(a.off[x + 1] - a.off[x]);
+        }
+#pragma unroll
+        for (int t = 0; t < 5; ++t) {
+          const uint32_t m = __ballot_sync(kFull, tier == t);
+          if (!m) continue;
+          uint32_t base = 0;
+          if (lane == __ffs(m) - 1) base = atomicAdd(f.tier[t].count, (uint32_t)__popc(m));
+          base = __shfl_sync(kFull, base, __ffs(m) - 1);
+          if (tier == t) f.tier[t].ids[base + __popc(m & ((1u << lane) - 1u))] = x;
+        }
+      }
+    }
+    return;
+  }
   for (int64_t i0 = 4 * (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); i0 < nc; i0 += 4 * nw) {
     const int64_t i = i0 + (lane >> 3);
     int32_t b = 0, d = 0;
@@ -1881,6 +1919,8 @@ __global__ void __launch_bounds__(256) k_frontier_list(StepArgs a, Frontier f, i
   if (step_mode(a) != kModeFrontier) return;
   __shared__ uint32_t cnt[5], base[5];
   const int lane = threadIdx.x & 31;
+  const uint32_t nc = *f.chg_in_n;
+  if (frontier_direct(a, nc)) nscan = 0;  // listed already
   for (int64_t v0 = (int64_t)blockIdx.x * kListRound; v0 < nscan; v0 += (int64_t)gridDim.x * kListRound) {  // block-uniform
     if (threadIdx.x < 5) cnt[threadIdx.x] = 0u;
     __syncthreads();
@@ -1894,10 +1934,7 @@ __global__ void __launch_bounds__(256) k_frontier_list(StepArgs a, Frontier f, i
 #pragma unroll
     for (int q = 0; q < kListItems; ++q) {
       const int64_t v = v0 + q * 256 + threadIdx.x;
-      if (tier[q] == 0) {
-        const int32_t d = a.off[v + 1] - a.off[v];
-        tier[q] = d <= f.tiny_max ? 0 : d <= f.g16_max ? 1 : d <= 32 ? 2 : d <= f.mid_max ? 3 : d <= f.big_max ? 4 : -1;
-      }
+      if (tier[q] == 0) tier[q] = f.tier_of(a.off[v + 1] - a.off[v]);
     }
 #pragma unroll
     for (int q = 0; q < kListItems; ++q) {
@@ -1921,7 +1958,6 @@ __global__ void __launch_bounds__(256) k_frontier_list(StepArgs a, Frontier f, i
     __syncthreads();  // base is read no more
   }
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
-  const uint32_t nc = *f.chg_in_n;
   for (int64_t i = t0; i < nc; i += nt) {
     const int32_t v = f.chg_in[i];
     if (f.act[v] != f.epoch) a.lout[v] = a.lin[v];
