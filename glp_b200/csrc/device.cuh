@@ -172,32 +172,11 @@ __device__ __forceinline__ Best block_max(Best b, Best* scratch) {
   return r;
 }
 
-// Open-addressing counter table (linear probing) in shared or global memory:
-// keys hold label+1 (0 = empty), vals the running count or weight sum.
-// insert() returns the count AFTER adding c; the largest value returned for a
-// key over all of its inserts is its final total, whatever the order.
-struct CountTable {
-  uint32_t* keys;
-  uint32_t* vals;
-  uint32_t mask;  // capacity - 1, capacity a power of two
-
-  __device__ __forceinline__ uint32_t insert(uint32_t key, uint32_t c, uint32_t* err) const {
-    uint32_t h = fmix32(key) & mask;
-    for (uint32_t probe = 0; probe <= mask; ++probe) {
-      uint32_t cur = keys[h];
-      if (cur == 0) {
-        uint32_t prev = atomicCAS(&keys[h], 0u, key);
-        if (prev == 0u || prev == key) return atomicAdd(&vals[h], c) + c;
-      } else if (cur == key) {
-        return atomicAdd(&vals[h], c) + c;
-      }
-      h = (h + 1) & mask;
-    }
-    atomicOr(err, kErrProbe);
-    return 0;
-  }
-};
-
+// Open-addressing counter tables: keys hold label+1 (0 = empty), vals the running
+// count or weight sum.  An insert returns the count AFTER adding c; the largest
+// value returned for a key over all of its inserts is its final total, whatever
+// the order.
+//
 // Bounded insert: gives up after `max_probe` probes and returns kNoSlot.
 // The home slot is the top bits of a Fibonacci (multiplicative) hash, one
 // multiply-high; on a collision the probe continues by double hashing with an
@@ -330,11 +309,5 @@ __device__ __forceinline__ void sort_keys(K (&x)[N]) {
 
 // Smallest power of two >= x (x >= 1).
 __device__ __forceinline__ uint32_t pow2_ceil(uint32_t x) { return x <= 1 ? 1u : 1u << (32 - __clz(x - 1)); }
-
-// Warp-aggregated add of per-lane counts (0..255) to a counter.
-__device__ __forceinline__ void warp_count_add(unsigned long long* counter, uint32_t count) {
-  const uint32_t total = __reduce_add_sync(kFull, count);
-  if ((threadIdx.x & 31) == 0 && total) atomicAdd(counter, (unsigned long long)total);
-}
 
 }  // namespace glp
