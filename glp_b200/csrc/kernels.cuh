@@ -1984,7 +1984,7 @@ __global__ void k_check_symmetric(const int32_t* __restrict__ off, const int32_t
     int32_t a = off[u], b = off[u + 1] - 1;
     bool found = false;
     while (a <= b) {
-      const int32_t mid = (a + b) >> 1;
+      const int32_t mid = a + (b - a) / 2;  // (a + b passes 2^31 in rows beyond 2^30)
       const int32_t x = cols[mid];
       if (x == v) {
         found = true;
