@@ -65,7 +65,7 @@ __global__ void k_cm_sketch(const int32_t* off, const int32_t* cols, const int32
     for (uint32_t s = threadIdx.x; s < cells; s += blockDim.x) rows[s] = 0;
     __syncthreads();
     const int32_t v = verts[i];
-    for (int32_t j = off[v] + threadIdx.x; j < off[v + 1]; j += blockDim.x) {
+    for (uint32_t j = off[v] + threadIdx.x; j < (uint32_t)off[v + 1]; j += blockDim.x) {
       const uint32_t key = (uint32_t)labels[cols[j]] + 1u;
       const uint32_t x = w ? (uint32_t)w[j] : 1u;
 #pragma unroll
@@ -165,21 +165,21 @@ __global__ void __launch_bounds__(NT) k_big_cm(StepArgs a, TierWork tw, S score,
     };
     Best best = best_none();
     bool fail = false;
-    for (int32_t j0 = b + warp * 32; j0 < e; j0 += 4 * NT) {
+    for (uint32_t j0 = b + warp * 32; j0 < (uint32_t)e; j0 += 4 * NT) {
       int32_t lab[4];
       uint32_t wt[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int32_t j = j0 + q * NT + lane;
-        lab[q] = j < e ? ld_stream(a.cols + j) : -1;
-        wt[q] = j < e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
+        const uint32_t j = j0 + q * NT + lane;
+        lab[q] = j < (uint32_t)e ? ld_stream(a.cols + j) : -1;
+        wt[q] = j < (uint32_t)e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         if (lab[q] >= 0) lab[q] = ld_label(a.lin + lab[q]);
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (j0 + q * NT < e) count_chunk<W>(lab[q] >= 0, lab[q], wt[q], score, ins, best, fail, true);
+        if (j0 + q * NT < (uint32_t)e) count_chunk<W>(lab[q] >= 0, lab[q], wt[q], score, ins, best, fail, true);
     }
     __syncthreads();
     scan_table(tkeys, tvals, kCmTable, threadIdx.x, NT, score, best);
@@ -378,20 +378,20 @@ __global__ void __launch_bounds__(NT) k_big_fa(StepArgs a, TierWork tw, S score,
     const int32_t v = tw.at(mode, i);
     const int32_t b = a.off[v], e = a.off[v + 1];
     FaSummary fs{skey[warp], sval[warp], splb[warp]};
-    for (int32_t j0 = b; j0 < e; j0 += 128) {
+    for (uint32_t j0 = b; j0 < (uint32_t)e; j0 += 128) {
       int32_t lab[4];
       uint32_t wt[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int32_t j = j0 + 32 * q + lane;
-        lab[q] = j < e ? ld_stream(a.cols + j) : -1;
-        wt[q] = j < e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
+        const uint32_t j = j0 + 32 * q + lane;
+        lab[q] = j < (uint32_t)e ? ld_stream(a.cols + j) : -1;
+        wt[q] = j < (uint32_t)e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) lab[q] = lab[q] >= 0 ? ld_label(a.lin + lab[q]) : INT32_MAX;
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (j0 + 32 * q < e) fs.add_chunk<W>(lab[q], wt[q]);
+        if (j0 + 32 * q < (uint32_t)e) fs.add_chunk<W>(lab[q], wt[q]);
     }
     const int32_t* ck = fs.key(fs.cur);
     uint32_t* cnt = fs.val(fs.cur);
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(NT) k_big_fa(StepArgs a, TierWork tw, S score,
       cnt = fs.val(fs.cur ^ 1);
       for (int32_t s = lane; s < fs.ns; s += 32) cnt[s] = 0u;
       __syncwarp();
-      for (int32_t j = b + lane; j < e; j += 32) {
+      for (uint32_t j = b + lane; j < (uint32_t)e; j += 32) {
         const int32_t l = ld_label(a.lin + ld_stream(a.cols + j));
         const int32_t p = lower_bound_keys(ck, fs.ns, l);
         if (p < fs.ns && ck[p] == l) atomicAdd(&cnt[p], W ? (uint32_t)ld_stream(a.w + j) : 1u);

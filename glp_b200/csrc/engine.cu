@@ -1663,19 +1663,19 @@ __global__ void __launch_bounds__(NT) k_noalloc_step(const int32_t* __restrict__
     auto ins = [&](uint32_t key, uint32_t k) {
       return table_insert_bounded(keys, vals, cap - 1, key, k, cap, nullptr, nullptr);
     };
-    for (int32_t j0 = b + warp * 32; j0 < e; j0 += 4 * NT) {
+    for (uint32_t j0 = b + warp * 32; j0 < (uint32_t)e; j0 += 4 * NT) {
       int32_t lab[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int32_t j = j0 + q * NT + lane;
-        lab[q] = j < e ? ld_stream(cols + j) : -1;
+        const uint32_t j = j0 + q * NT + lane;
+        lab[q] = j < (uint32_t)e ? ld_stream(cols + j) : -1;
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         if (lab[q] >= 0) lab[q] = ld_label(lin + lab[q]);
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (j0 + q * NT < e) count_chunk<false>(lab[q] >= 0, lab[q], 1u, score, ins, best, fail);
+        if (j0 + q * NT < (uint32_t)e) count_chunk<false>(lab[q] >= 0, lab[q], 1u, score, ins, best, fail);
     }
     if (fail) atomicOr(err, kErrProbe);
     best = block_max<NT>(best, red);

@@ -53,7 +53,9 @@ struct BigBound {
   __device__ __forceinline__ bool has(int32_t v) const { return (uint32_t)(v - base) < (uint32_t)n; }
 };
 
-// Neighbour labels, own labels and the output of one step.
+// Neighbour labels, own labels and the output of one step.  (Kernels count a
+// row's entries from its start, or by uint32_t: the rounds of the last row of a
+// graph of almost 2^31 entries go past 2^31.)
 struct StepArgs {
   const int32_t* off;
   const int32_t* cols;
@@ -701,15 +703,14 @@ __global__ void __launch_bounds__(256) k_major_warp(StepArgs a, Verts vs, int32_
     // after the whole row, and a formed community's big rows are decided
     // after a little more than half of their entries
     const uint32_t d = (uint32_t)(e - b);
-    for (int32_t c0 = b; c0 < e; c0 += 32 * U) {  // warp-uniform chunks
-      const int32_t j0 = c0 + lane;
+    for (int32_t c0 = 0; c0 < e - b; c0 += 32 * U) {  // warp-uniform chunks
       int32_t c[U];
       uint32_t wt[U];
 #pragma unroll
       for (int q = 0; q < U; ++q) {
-        const int32_t j = j0 + 32 * q;
-        c[q] = j < e ? ld_stream(a.cols + j) : -1;
-        wt[q] = j < e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
+        const int32_t i = c0 + lane + 32 * q;
+        c[q] = i < e - b ? ld_stream(a.cols + (b + i)) : -1;
+        wt[q] = i < e - b ? (W ? (uint32_t)ld_stream(a.w + (b + i)) : 1u) : 0u;
       }
 #pragma unroll
       for (int q = 0; q < U; ++q) {
@@ -717,8 +718,8 @@ __global__ void __launch_bounds__(256) k_major_warp(StepArgs a, Verts vs, int32_
         cnt += l == cand ? wt[q] : 0u;
         tot += wt[q];
       }
-      if (!W && c0 + 32 * U < e) {
-        const uint32_t seen = (uint32_t)(c0 + 32 * U - b);
+      if (!W && c0 + 32 * U < e - b) {
+        const uint32_t seen = (uint32_t)(c0 + 32 * U);
         const uint32_t sc = __reduce_add_sync(kFull, cnt);
         if (2ull * sc > d || 2ull * (sc + (d - seen)) <= d) {
           cnt = lane == 0 ? sc : 0u;  // the reduction below returns sc
@@ -783,14 +784,14 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
   const bool merge = !CF || mode != kModeFull || S::kMajority || S::kKeep;
   uint32_t* kk = skeys[warp];
   uint32_t* vv = svals[warp];
-  // batch loader: columns (and weights) of entries j0 + 32q + lane below e,
+  // batch loader: columns (and weights) of the row's entries i0 + 32q + lane,
   // then their labels (-1 past the row)
-  auto load_batch = [&](int32_t j0, int32_t e, int32_t (&lab)[4], uint32_t (&wt)[4], int32_t (&vl)[4]) {
+  auto load_batch = [&](int32_t b, int32_t i0, int32_t d, int32_t (&lab)[4], uint32_t (&wt)[4], int32_t (&vl)[4]) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int32_t j = j0 + 32 * q + lane;
-      lab[q] = j < e ? ld_stream(a.cols + j) : -1;
-      wt[q] = j < e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
+      const int32_t i = i0 + 32 * q + lane;
+      lab[q] = i < d ? ld_stream(a.cols + (b + i)) : -1;
+      wt[q] = i < d ? (W ? (uint32_t)ld_stream(a.w + (b + i)) : 1u) : 0u;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -806,7 +807,7 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
       pb = a.off[pv];
       pe = a.off[pv + 1];
     }
-    load_batch(pb, pe, plab, pwt, pvl);
+    load_batch(pb, 0, pe - pb, plab, pwt, pvl);
   };
   int32_t i = blockIdx.x * NW + warp;
   if (PF) prefetch(i);
@@ -849,10 +850,10 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
                 : table_insert_bounded<C16>(kk, vv, cap - 1, key, k, cap, nullptr, nullptr);
     };
     ChunkQueue<W> queue(&rings[RING ? warp : 0]);
-    for (int32_t j0 = b; j0 < e; j0 += 128) {
+    for (int32_t i0 = 0; i0 < e - b; i0 += 128) {
       int32_t lab[4], vl[4];
       uint32_t wt[4];
-      if (PF && j0 == b) {
+      if (PF && i0 == 0) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           lab[q] = lab0[q];
@@ -860,19 +861,19 @@ __global__ void __launch_bounds__(NT, PF ? (S::kPacked ? 1536 : 1024) / NT
           vl[q] = vl0[q];
         }
       } else {
-        load_batch(j0, e, lab, wt, vl);
+        load_batch(b, i0, e - b, lab, wt, vl);
       }
       if constexpr (RING) {
         if (score.single) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            if (j0 + 32 * q < e) queue.add(lab[q] >= 0, lab[q], wt[q], vl[q], score, ins, best, fail, scan, merge);
+            if (i0 + 32 * q < e - b) queue.add(lab[q] >= 0, lab[q], wt[q], vl[q], score, ins, best, fail, scan, merge);
           continue;
         }
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (j0 + 32 * q < e)
+        if (i0 + 32 * q < e - b)
           count_chunk<W, S::kLV>(lab[q] >= 0, lab[q], wt[q], score, ins, best, fail, scan, vl[q], merge);
     }
     if constexpr (RING) queue.finish(score, ins, best, fail, scan, merge);
@@ -998,14 +999,14 @@ __global__ void __launch_bounds__(NT, (!W ? (NT == 1024 && S::kPacked ? (S::kLV 
         continue;
       }
       uint32_t cnt = 0, tot = 0;
-      for (int32_t j0 = b + threadIdx.x; j0 < e; j0 += 4 * NT) {
+      for (uint32_t j0 = b + threadIdx.x; j0 < (uint32_t)e; j0 += 4 * NT) {
         int32_t c[4];
         uint32_t wt[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int32_t j = j0 + q * NT;
-          c[q] = j < e ? ld_stream(a.cols + j) : -1;
-          wt[q] = j < e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
+          const uint32_t j = j0 + q * NT;
+          c[q] = j < (uint32_t)e ? ld_stream(a.cols + j) : -1;
+          wt[q] = j < (uint32_t)e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -1059,14 +1060,14 @@ __global__ void __launch_bounds__(NT, (!W ? (NT == 1024 && S::kPacked ? (S::kLV 
     // lanes' adds to one slot serialise
     const bool merge = !CF || mode != kModeFull || (e - b) > kMergeDegree || S::kKeep;
     ChunkQueue<W> queue(&rings[S::kLV ? warp : 0]);
-    for (int32_t j0 = b + warp * 32; j0 < e; j0 += 4 * NT) {
+    for (uint32_t j0 = b + warp * 32; j0 < (uint32_t)e; j0 += 4 * NT) {
       int32_t lab[4], vl[4];
       uint32_t wt[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int32_t j = j0 + q * NT + lane;
-        lab[q] = j < e ? ld_stream(a.cols + j) : -1;
-        wt[q] = j < e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
+        const uint32_t j = j0 + q * NT + lane;
+        lab[q] = j < (uint32_t)e ? ld_stream(a.cols + j) : -1;
+        wt[q] = j < (uint32_t)e ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
@@ -1075,13 +1076,13 @@ __global__ void __launch_bounds__(NT, (!W ? (NT == 1024 && S::kPacked ? (S::kLV 
         if (score.single) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            if (j0 + q * NT < e) queue.add(lab[q] >= 0, lab[q], wt[q], vl[q], score, ins, best, fail, scan, merge);
+            if (j0 + q * NT < (uint32_t)e) queue.add(lab[q] >= 0, lab[q], wt[q], vl[q], score, ins, best, fail, scan, merge);
           continue;
         }
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (j0 + q * NT < e)
+        if (j0 + q * NT < (uint32_t)e)
           count_chunk<W, S::kLV>(lab[q] >= 0, lab[q], wt[q], score, ins, best, fail, scan, vl[q], merge);
     }
     if constexpr (S::kLV) queue.finish(score, ins, best, fail, scan, merge);
@@ -1156,8 +1157,8 @@ __global__ void __launch_bounds__(NT, S::kSMThreads / NT) k_big_staged(StepArgs 
   // thread 0: stage the row of work item idx into buffer bi
   auto issue = [&](int32_t idx, int bi) {
     const int32_t u = tw.at(mode, idx);
-    const int32_t lo = a.off[u] & ~3, hi = (a.off[u + 1] + 3) & ~3;
-    const uint32_t bytes = (uint32_t)(hi - lo) * 4u;
+    const uint32_t lo = (uint32_t)a.off[u] & ~3u, hi = ((uint32_t)a.off[u + 1] + 3u) & ~3u;
+    const uint32_t bytes = (hi - lo) * 4u;
     fence_proxy_async_smem();
     mbar_arrive_expect_tx(&bar[bi], bytes);
     bulk_copy_g2s(scol[bi], a.cols + lo, bytes, &bar[bi]);
@@ -1194,12 +1195,12 @@ __global__ void __launch_bounds__(NT, S::kSMThreads / NT) k_big_staged(StepArgs 
       }
     }
     ph[bi] ^= 1u;
-    const int32_t lo = b & ~3;
+    const uint32_t lo = (uint32_t)b & ~3u;
     int32_t lab[ITEMS], vl[ITEMS];
 #pragma unroll
     for (int q = 0; q < ITEMS; ++q) {
-      const int32_t j = b + q * NT + (int32_t)threadIdx.x;
-      lab[q] = j < e ? scol[bi][j - lo] : -1;
+      const uint32_t j = (uint32_t)b + q * NT + threadIdx.x;
+      lab[q] = j < (uint32_t)e ? scol[bi][j - lo] : -1;
     }
 #pragma unroll
     for (int q = 0; q < ITEMS; ++q)
@@ -1209,7 +1210,7 @@ __global__ void __launch_bounds__(NT, S::kSMThreads / NT) k_big_staged(StepArgs 
     auto ins = [&](uint32_t key, uint32_t k) { return table_claim_insert<true>(keys, vals, cap - 1, key, k, cap); };
 #pragma unroll
     for (int q = 0; q < ITEMS; ++q)
-      if (b + q * NT + (threadIdx.x & ~31u) < (uint32_t)e)  // warp-uniform
+      if ((uint32_t)b + q * NT + (threadIdx.x & ~31u) < (uint32_t)e)  // warp-uniform
         count_chunk<false, S::kLV>(lab[q] >= 0, lab[q], 1u, score, ins, best, fail, scan, vl[q], false);
     if (fail) atomicOr(a.err, kErrProbe);
     if (scan) {  // block-uniform
@@ -1337,14 +1338,14 @@ __global__ void __launch_bounds__(NT) k_hub_majority(StepArgs a, HubPlan hp, int
     const int32_t cand = a.lcur[hp.hub_v[h]];
     const int32_t cb = hp.chunk_begin[c], ce = hp.chunk_end[c];
     uint32_t cnt = 0, tot = 0;
-    for (int32_t j0 = cb + threadIdx.x; j0 < ce; j0 += 8 * NT) {
+    for (uint32_t j0 = cb + threadIdx.x; j0 < (uint32_t)ce; j0 += 8 * NT) {
       int32_t col[8];
       uint32_t wt[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const int32_t j = j0 + q * NT;
-        col[q] = j < ce ? ld_stream(a.cols + j) : -1;
-        wt[q] = j < ce ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
+        const uint32_t j = j0 + q * NT;
+        col[q] = j < (uint32_t)ce ? ld_stream(a.cols + j) : -1;
+        wt[q] = j < (uint32_t)ce ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
       }
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
@@ -1410,14 +1411,14 @@ __global__ void __launch_bounds__(NT) k_hub_gather(StepArgs a, HubPlan hp, int32
     for (uint32_t b = threadIdx.x; b < nb; b += NT) hist[b] = 0;
     __syncthreads();
     Best alone = best_none();
-    for (int32_t j0 = cb + threadIdx.x; j0 < ce; j0 += 4 * NT) {
+    for (uint32_t j0 = cb + threadIdx.x; j0 < (uint32_t)ce; j0 += 4 * NT) {
       int32_t col[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) col[q] = j0 + q * NT < ce ? ld_stream(a.cols + j0 + q * NT) : -1;
+      for (int q = 0; q < 4; ++q) col[q] = j0 + q * NT < (uint32_t)ce ? ld_stream(a.cols + (j0 + q * NT)) : -1;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         if (col[q] < 0) continue;
-        const int32_t j = j0 + q * NT;
+        const uint32_t j = j0 + q * NT;
         int32_t l = -1, vl = 0;
         const int32_t w = W ? ld_stream(a.w + j) : 1;
         if constexpr (S::kLV) {
@@ -1682,10 +1683,10 @@ __global__ void k_cycle_end(const int32_t* __restrict__ chg, const uint32_t* n_n
 // (unweighted).
 __global__ void __launch_bounds__(256) k_first_step(StepArgs a) {
   ChangeNotes notes(a);
-  for (int32_t v0 = blockIdx.x * blockDim.x; v0 < a.n; v0 += gridDim.x * blockDim.x) {
-    const int32_t v = v0 + threadIdx.x;
+  for (int64_t v0 = (int64_t)blockIdx.x * blockDim.x; v0 < a.n; v0 += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t v = (int32_t)(v0 + threadIdx.x);  // (negative past 2^31)
     bool chg = false;
-    if (v < a.n) {
+    if (v0 + threadIdx.x < a.n) {
       const int32_t e = a.off[v + 1];
       if (e > a.off[v]) {
         const int32_t l = a.lin[a.cols[e - 1]];
@@ -1704,7 +1705,7 @@ __global__ void __launch_bounds__(256) k_first_step(StepArgs a) {
 // hubs go to k_first_step_w_block.  The key of an entry is
 // a 64-bit word monotone in (score, label) and never 0 for a candidate.
 struct FirstKeyW {
-  __device__ __forceinline__ unsigned long long operator()(const StepArgs& a, int32_t j) const {
+  __device__ __forceinline__ unsigned long long operator()(const StepArgs& a, uint32_t j) const {
     return ((unsigned long long)(uint32_t)a.w[j] << 32) | (uint32_t)a.lin[a.cols[j]];
   }
 };
@@ -1716,7 +1717,7 @@ template <bool W>
 struct FirstKeyLayered {
   const int32_t* vol;
   int32_t dstar;
-  __device__ __forceinline__ unsigned long long operator()(const StepArgs& a, int32_t j) const {
+  __device__ __forceinline__ unsigned long long operator()(const StepArgs& a, uint32_t j) const {
     const int32_t l = ld_stream(a.cols + j);
     const int32_t k = W ? ld_stream(a.w + j) : 1;
     const int32_t sc = dstar * k - __ldg(vol + l);
@@ -1737,16 +1738,16 @@ __global__ void __launch_bounds__(256) k_first_step_w(StepArgs a, Verts vs, K ke
       const int32_t b = a.off[v], e = a.off[v + 1];
       if (G == 1) {
         // eight entries a round, their loads in flight together
-        for (int32_t j0 = b; j0 < e; j0 += 8) {
+        for (uint32_t j0 = b; j0 < (uint32_t)e; j0 += 8) {
 #pragma unroll
           for (int q = 0; q < 8; ++q)
-            if (j0 + q < e) best = max(best, key(a, j0 + q));
+            if (j0 + q < (uint32_t)e) best = max(best, key(a, j0 + q));
         }
       } else {
-        for (int32_t j0 = b + lane; j0 < e; j0 += 4 * G) {
+        for (uint32_t j0 = b + lane; j0 < (uint32_t)e; j0 += 4 * G) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            if (j0 + q * G < e) best = max(best, key(a, j0 + q * G));
+            if (j0 + q * G < (uint32_t)e) best = max(best, key(a, j0 + q * G));
         }
       }
     }
@@ -1770,10 +1771,10 @@ __global__ void __launch_bounds__(NT) k_first_step_w_block(StepArgs a, Verts vs,
     if (threadIdx.x == 0) sb = 0ull;
     __syncthreads();
     unsigned long long best = 0ull;
-    for (int32_t j0 = b + threadIdx.x; j0 < e; j0 += 4 * NT) {
+    for (uint32_t j0 = b + threadIdx.x; j0 < (uint32_t)e; j0 += 4 * NT) {
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (j0 + q * NT < e) best = max(best, key(a, j0 + q * NT));
+        if (j0 + q * NT < (uint32_t)e) best = max(best, key(a, j0 + q * NT));
     }
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) best = max(best, __shfl_xor_sync(kFull, best, m));
@@ -1797,11 +1798,11 @@ __global__ void __launch_bounds__(256) k_check_sorted(const int32_t* __restrict_
   for (int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += nw) {
     const int32_t b = off[v], e = off[v + 1];
     bool ok = true;
-    for (int32_t j0 = b + 1 + lane; j0 < e; j0 += 256) {
+    for (uint32_t j0 = (uint32_t)b + 1u + lane; j0 < (uint32_t)e; j0 += 256) {
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const int32_t j = j0 + 32 * q;
-        if (j < e && ld_stream(cols + j - 1) >= ld_stream(cols + j)) ok = false;
+        const uint32_t j = j0 + 32 * q;
+        if (j < (uint32_t)e && ld_stream(cols + j - 1) >= ld_stream(cols + j)) ok = false;
       }
     }
     if (__any_sync(kFull, !ok) && lane == 0) atomicOr(bad, 1u);
@@ -2014,7 +2015,7 @@ __global__ void __launch_bounds__(256) k_histogram(const int32_t* __restrict__ l
 // one 8-byte load per neighbour (ScoreLayered32::load).
 __global__ void __launch_bounds__(256) k_label_volumes(const int32_t* __restrict__ lab, const int32_t* __restrict__ vol,
                                                        int32_t n, int2* __restrict__ lv) {
-  for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
     const int32_t l = lab[v];
     lv[v] = make_int2(l, __ldg(vol + l));
   }
