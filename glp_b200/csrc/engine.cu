@@ -363,28 +363,32 @@ static int ensure_plan(glp_graph* g, const TierParams& t) {
     p.merged = p.small && t.tiny_auto;
     build_host_plan(g->h_off.data(), g->n, t, &hp, p.merged);
     p.isolated = hp.isolated;
-    if ((rc = upload_verts(&p, hp.tiny, &p.tiny)) || (rc = upload_verts(&p, hp.g16, &p.g16)) ||
-        (rc = upload_verts(&p, hp.g32, &p.g32)) || (rc = upload_verts(&p, hp.mid, &p.mid)) ||
-        (rc = upload_verts(&p, hp.big, &p.big)) || (rc = upload_verts(&p, hp.mb, &p.mb)) ||
-        (rc = upload_verts(&p, hp.pair, &p.pair)) || (rc = upload_verts(&p, hp.mid_rest, &p.mid_rest)) ||
-        (rc = upload_verts(&p, hp.mb_rest, &p.mb_rest))) {
-      free_plan(&p);
-      return rc;
+    // the lists that the graph's scores use: mb of weighted classic, the pair
+    // rows and the tiers without them of unweighted classic-type scores, the
+    // merged big ranges of few big vertices
+    std::vector<int32_t> low = merge_ids(hp.big_part[0], hp.big_part[1]);
+    std::vector<std::pair<const std::vector<int32_t>*, Verts*>> lists = {
+        {&hp.tiny, &p.tiny}, {&hp.g16, &p.g16}, {&hp.g32, &p.g32}, {&hp.mid, &p.mid}, {&hp.big, &p.big}};
+    if (g->d_w) {
+      lists.push_back({&hp.mb, &p.mb});
+    } else {
+      lists.push_back({&hp.pair, &p.pair});
+      lists.push_back({&hp.mid_rest, &p.mid_rest});
+      lists.push_back({&hp.mb_rest, &p.mb_rest});
     }
-    for (int r = 0; r < kBigParts; ++r)
-      if ((rc = upload_verts(&p, hp.big_part[r], &p.big_part[r]))) {
+    for (int r = 0; r < kBigParts; ++r) lists.push_back({&hp.big_part[r], &p.big_part[r]});
+    lists.push_back({&low, &p.big_first});
+    for (const auto& l : lists)
+      if ((rc = upload_verts(&p, *l.first, l.second))) {
         free_plan(&p);
         return rc;
       }
-    std::vector<int32_t> low = merge_ids(hp.big_part[0], hp.big_part[1]);
-    if ((rc = upload_verts(&p, low, &p.big_first))) {
-      free_plan(&p);
-      return rc;
-    }
-    for (int r = 2; r < kBigLowParts; ++r) low = merge_ids(low, hp.big_part[r]);
-    if ((rc = upload_verts(&p, low, &p.big_low))) {
-      free_plan(&p);
-      return rc;
+    if (p.big.n <= kFewBig) {
+      for (int r = 2; r < kBigLowParts; ++r) low = merge_ids(low, hp.big_part[r]);
+      if ((rc = upload_verts(&p, low, &p.big_low))) {
+        free_plan(&p);
+        return rc;
+      }
     }
   }
   n_mid = p.mid.n;
@@ -884,7 +888,7 @@ struct RunCtx {
       ran.back()[3] = p.mid.n > 0;
       ran.back()[4] = p.big.n > 0;
       ran.back()[5] = p.n_hubs > 0;
-      ran.back()[7] = p.mb.n > 0;
+      ran.back()[7] = p.mb.n > 0 || p.mb_rest.n > 0;
       ran.back()[8] = true;
     }
     StepLaunch L{&g->plan, s, ev, {g->aux[0], g->aux[1]}, g->fork, {g->join[0], g->join[1]}};
