@@ -601,6 +601,30 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
   const bool late = W && S::kLV && (int64_t)a.n * (int64_t)sizeof(int2) > device_l2();
   if (!late) GLP_CUDA(cudaStreamWaitEvent(L.aux[1], L.fork, 0));
   constexpr int kMidNT = 256, kBigNT = 256, kHubNT = 512, kBucketNT = 512;
+  // On graphs whose labels outgrow a quarter of the L2 the hubs' scatter and
+  // count follow the big tier, beside the mid tier: which of them the device
+  // starts first is otherwise a matter of the streams' hardware queues, and
+  // k_mid on SMs that k_hub_bucket's 64 KB blocks share takes 1.2 ms instead of
+  // 0.9 (R-MAT s24, 20 steps: 17.6 or 16.8 ms by the handle, now 17.2; weighted
+  // 78.4 -> 75.7, layered weighted 309 -> 303; s23 10.9 and 11.0, weighted 33.2 ->
+  // 32.5).  Smaller graphs want the overlap (s22 6.0 -> 6.2), and so do unweighted
+  // layered scores (s24 185 -> 188).
+  const bool hubs_late = p.n_hubs && p.big.n && p.mid.n && !L.ev && (W || !S::kLV) &&
+                         (int64_t)a.n * (int64_t)sizeof(int32_t) > device_l2() / 4;
+  auto hub_scatter = [&] {
+    const unsigned grid = (unsigned)std::min<int64_t>(p.n_chunks, kMaxGrid);
+    k_hub_scatter<kHubNT, W><<<grid, kHubNT, 2 * p.hub.max_nb * sizeof(uint32_t), L.aux[0]>>>(a, p.hub, p.n_chunks);
+  };
+  auto hub_count = [&]() -> int {
+    const size_t sm = 2ull * kHubTable * sizeof(uint32_t);
+    k_hub_bucket<kBucketNT, W, S><<<(unsigned)std::min<int64_t>(p.hub.nitems, device_sms() * 8), kBucketNT, sm, L.aux[0]>>>(
+        a, p.hub, score);
+    const uint8_t* seeds = nullptr;
+    if constexpr (S::kKeep) seeds = score.seeds;
+    k_hub_finalize<<<(unsigned)cdiv(p.n_hubs, 256), 256, 0, L.aux[0]>>>(a, p.hub, seeds);
+    *launches += 6;
+    return mark_on(L.aux[0], 5, 1);
+  };
   if (p.n_hubs) {
     const size_t sm = 2ull * kHubTable * sizeof(uint32_t);
     const size_t sm_hist = (size_t)p.hub.max_nb * sizeof(uint32_t);
@@ -619,14 +643,10 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     GLP_CUDA(cudaMemsetAsync(p.hub.bcnt, 0, sizeof(uint32_t) * p.hub.nitems, L.aux[0]));
     k_hub_gather<kHubNT, W, S><<<grid, kHubNT, sm_hist, L.aux[0]>>>(a, p.hub, p.n_chunks, score);
     k_hub_offsets<<<hgrid, 256, 0, L.aux[0]>>>(p.hub);
-    k_hub_scatter<kHubNT, W><<<grid, kHubNT, 2 * sm_hist, L.aux[0]>>>(a, p.hub, p.n_chunks);
-    k_hub_bucket<kBucketNT, W, S><<<(unsigned)std::min<int64_t>(p.hub.nitems, device_sms() * 8), kBucketNT, sm, L.aux[0]>>>(
-        a, p.hub, score);
-    const uint8_t* seeds = nullptr;
-    if constexpr (S::kKeep) seeds = score.seeds;
-    k_hub_finalize<<<hgrid, 256, 0, L.aux[0]>>>(a, p.hub, seeds);
-    *launches += 6;
-    if ((rc = mark_on(L.aux[0], 5, 1))) return rc;
+    if (!hubs_late) {
+      hub_scatter();
+      if ((rc = hub_count())) return rc;
+    }
   }
   // unweighted classic-type scores count the mid tier's rows up to kPairDegree
   // by k_pair in full and majority steps
@@ -761,9 +781,14 @@ int launch_step(const StepLaunch& Lin, const StepArgs& a, const S& score, int64_
     }
     if ((rc = mark_on(s, 4, 1))) return rc;
   }
-  if (late) {
+  if (late || hubs_late) {
     GLP_CUDA(cudaEventRecord(L.fork, s));
-    GLP_CUDA(cudaStreamWaitEvent(L.aux[1], L.fork, 0));
+    if (late) GLP_CUDA(cudaStreamWaitEvent(L.aux[1], L.fork, 0));
+    if (hubs_late) {
+      GLP_CUDA(cudaStreamWaitEvent(L.aux[0], L.fork, 0));
+      hub_scatter();
+      if ((rc = hub_count())) return rc;
+    }
   }
   if (p.mid.n) {
     if ((rc = mark_on(s, 3, 0))) return rc;

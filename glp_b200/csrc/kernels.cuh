@@ -1701,8 +1701,8 @@ __global__ void __launch_bounds__(256) k_first_step(StepArgs a) {
 
 // The weighted form of the same shortcut: every neighbour label occurs once,
 // so its count is the edge's weight, and the step takes the neighbour label
-// of largest (weight, label).  G lanes per vertex (1 or 32); the rows of the
-// hubs go to k_first_step_w_block.  The key of an entry is
+// of largest (weight, label).  G lanes per vertex (1, 8 or 32); large
+// rows go to k_first_step_w_block.  The key of an entry is
 // a 64-bit word monotone in (score, label) and never 0 for a candidate.
 struct FirstKeyW {
   __device__ __forceinline__ unsigned long long operator()(const StepArgs& a, uint32_t j) const {

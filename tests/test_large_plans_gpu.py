@@ -161,3 +161,15 @@ def test_tiny_max_selects_the_small_tiers(order):
         tiny, group16, group32 = r.step_tier_ms[2][:3]
         assert group32 > 0
         assert (tiny > 0) == (t > 0) and (group16 > 0) == (t != 0), (t, tiny, group16)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_classic_labels_beyond_the_cache(weighted):
+    """Labels past a quarter of the L2: the hubs are counted after the big tier."""
+    l2 = torch.cuda.get_device_properties(0).L2_cache_size
+    off, cols = _graph("sorted", isolated=l2 // 16 + 1000)
+    w = _weights(off, cols) if weighted else None
+    with Graph(from_numpy(off, cols, w)) as g:
+        for niter in (2, 5):
+            got = g.run(_lib.METHOD_CLASSIC, niter, make_params(majority_permille=1, frontier_permille=-1))
+            np.testing.assert_array_equal(got.labels, O.classic_run(off, cols, niter, w=w))
