@@ -708,9 +708,10 @@ __global__ void __launch_bounds__(256) k_major_warp(StepArgs a, Verts vs, int32_
       uint32_t wt[U];
 #pragma unroll
       for (int q = 0; q < U; ++q) {
-        const int32_t i = c0 + lane + 32 * q;
-        c[q] = i < e - b ? ld_stream(a.cols + (b + i)) : -1;
-        wt[q] = i < e - b ? (W ? (uint32_t)ld_stream(a.w + (b + i)) : 1u) : 0u;
+        const bool in = c0 + lane < e - b - 32 * q;
+        const int64_t j = (int64_t)b + c0 + lane + 32 * q;
+        c[q] = in ? ld_stream(a.cols + j) : -1;
+        wt[q] = in ? (W ? (uint32_t)ld_stream(a.w + j) : 1u) : 0u;
       }
 #pragma unroll
       for (int q = 0; q < U; ++q) {
